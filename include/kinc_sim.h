@@ -195,7 +195,9 @@ int32_t kinc_sim_last_launch_count(const kinc_sim_ctx* ctx);
  *   prefetch       0, 4, 8 or 16: samples ahead the clustering sweeps (GMM EM passes,
  *                  K-means Lloyd and log-likelihood passes) prefetch into L2
  * Pearson without clustering (clusmethod none, corrmethod pearson) runs one thread
- * per pair and takes no shape.
+ * per pair and takes no shape; neither do the blocks that run GMM with one warp per
+ * pair (up to 5 clusters; blocks that do not fill the tile kernel's waves well enough
+ * to make up for its slower samples).
  */
 typedef struct kinc_sim_launch
 {

@@ -30,6 +30,7 @@ UNITS = [
     ("kinc_sim.cu", ["--fmad=false"]),
     ("sim_none.cu", ["--fmad=false"]),
     ("sim_gmm.cu", ["--fmad=false"]),
+    ("sim_gmm_pair.cu", ["--fmad=false"]),
     ("sim_kmeans.cu", ["--fmad=false"]),
     ("pearson_gemm.cu", []),
     ("compact.cu", []),

@@ -74,6 +74,20 @@ __global__ void k_masks(const float* __restrict__ gem, int32_t G, int32_t S, int
    }
 }
 
+/* largest usable-sample count of a gene, an upper bound of every pair's N, into *most */
+__global__ void k_most_usable(const uint32_t* __restrict__ umask, int32_t G, int32_t W, int* __restrict__ most)
+{
+   const int lane = threadIdx.x & 31;
+   int best = 0;
+   for ( int g = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); g < G; g += (int)((gridDim.x * blockDim.x) >> 5) )
+   {
+      int n = 0;
+      for ( int w = lane; w < W; w += 32 ) n += __popc(umask[(size_t)g * W + w]);
+      best = max(best, __reduce_add_sync(0xffffffffu, n));
+   }
+   if ( lane == 0 ) atomicMax(most, best);
+}
+
 __device__ __forceinline__ int pair_count(const uint32_t* __restrict__ umask, int W, int64_t p)
 {
    int32_t x, y;
@@ -320,6 +334,10 @@ struct kinc_sim_ctx
    int smem_warp = 0;               /* dynamic shared memory per warp */
    int sms = 0;
    int64_t slots = 0;               /* warp scratch slots allocated */
+   int n_cap = 0;                   /* no pair has more usable samples */
+   int gmm_per_sm = 0;              /* GMM with one warp per pair (sim_gmm_pair.cuh): pairs an SM holds, 0: not available */
+   int64_t gmm_wave = 0;            /* pairs the tile kernel runs at once */
+   DevScratch dsp {};               /* its scratch */
    kinc_sim_launch launch {};
    char gpu_name[256] = "";
    int64_t max_block = 0;
@@ -345,6 +363,7 @@ struct kinc_sim_ctx
    int8_t* d_labels = nullptr;
    float* d_corr = nullptr;
    void* d_scratch = nullptr;
+   void* d_pairs = nullptr;
    /* host-side tracking of the rand() position held in d_qbase */
    int64_t q_valid_end = 0;
    int32_t launches = 0;
@@ -546,7 +565,7 @@ static void release(kinc_sim_ctx* c)
 {
    void* ptrs[] = { c->d_gem, c->d_umask, c->d_logn, c->d_jump, c->d_rng0, c->d_N, c->d_pg, c->d_qpos,
                     c->d_bsum, c->d_qbase, c->d_tiles, c->d_work, c->d_compact, c->d_order, c->d_bins, c->d_status, c->d_K, c->d_labels, c->d_corr,
-                    c->d_scratch };
+                    c->d_scratch, c->d_pairs };
    for ( void* p : ptrs )
       if ( p ) cudaFree(p);
    tc_release(c->tc);
@@ -751,9 +770,28 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
       grid -= prop.multiProcessorCount;
    const size_t slots = (size_t)grid * wpb;
    ctx->sms = prop.multiProcessorCount;
+   CKC(cudaMalloc(&ctx->d_status, sizeof(int)));
+   ctx->n_cap = S;
+   if ( params->clus_method == 1 )
+   {
+      CKC(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
+      k_most_usable<<<std::min((genes + 7) / 8, 1024), 256, 0, ctx->stream>>>(ctx->d_umask, genes, W, ctx->d_status);
+      CKC(cudaGetLastError());
+      CKC(cudaMemcpyAsync(&ctx->n_cap, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      CKC(cudaStreamSynchronize(ctx->stream));
+      ctx->gmm_per_sm = sim_gmm_pairs_per_sm(dp, ctx->n_cap);
+      ctx->gmm_wave = (int64_t)slots * TILE;
+   }
    snprintf(ctx->gpu_name, sizeof ctx->gpu_name, "%s", prop.name);
    ctx->slots = (int64_t)slots;
    ctx->smem_warp = (int)((ctx->smem_sort ? sort_bytes_warp : 0) + param_bytes_warp);
+   if ( ctx->gmm_per_sm > 0 )
+   {
+      CKC(cudaMalloc(&ctx->d_pairs, sim_gmm_pairs_scratch(ctx->sms, dp, ctx->n_cap, nullptr, ctx->dsp)));
+      sim_gmm_pairs_scratch(ctx->sms, dp, ctx->n_cap, (char*)ctx->d_pairs, ctx->dsp);
+   }
+   /* a whole wave is the tile kernel's best case: without one, nothing runs there */
+   if ( !sim_gmm_pairs_better(ctx->gmm_per_sm, ctx->gmm_wave, ctx->gmm_wave) )
    {
       size_t off = 0;
       auto take = [&](size_t bytes) {
@@ -817,7 +855,6 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
       CKC(cudaMalloc(&ctx->d_bins, ctx->nbins * sizeof(unsigned int)));
    }
    CKC(cudaMemsetAsync(ctx->d_work, 0, 4 * sizeof(unsigned long long), ctx->stream));
-   CKC(cudaMalloc(&ctx->d_status, sizeof(int)));
    CKC(cudaMalloc(&ctx->d_K, ctx->max_block));
    if ( params->precision == 0 ) CKC(cudaMalloc(&ctx->d_labels, (size_t)ctx->max_block * S));
    CKC(cudaMalloc(&ctx->d_corr, (size_t)ctx->max_block * params->max_clusters * dp.ncorr * sizeof(float)));
@@ -934,6 +971,10 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
    if ( lanes )
    {
       CK(sim_launch_pearson_lanes(ctx->sms, st, dp, ctx->dd, B));
+   }
+   else if ( sim_gmm_pairs_better(ctx->gmm_per_sm, size, ctx->gmm_wave) )
+   {
+      CK(sim_launch_gmm_pairs(ctx->sms, st, dp, ctx->dd, ctx->dsp, B, ctx->n_cap));
    }
    else
    {
