@@ -192,8 +192,8 @@ int32_t kinc_sim_last_launch_count(const kinc_sim_ctx* ctx);
  *   rounds         1: a CTA's warps take their 32-pair tiles together, round by
  *                  round (they then run the same code region at the same time);
  *                  0: every warp takes its next tile as soon as it is done
- *   prefetch       0, 4, 8 or 16: samples ahead the clustering sweeps (GMM EM passes,
- *                  K-means Lloyd and log-likelihood passes) prefetch into L2
+ *   prefetch       0, 4, 8 or 16: samples ahead the GMM EM passes prefetch into L2
+ * K-means up to 5 clusters takes only warps_per_cta (its warps work apart).
  * Pearson without clustering (clusmethod none, corrmethod pearson) runs one thread
  * per pair and takes no shape; neither do the blocks that run GMM with one warp per
  * pair (up to 5 clusters; blocks that do not fill the tile kernel's waves well enough

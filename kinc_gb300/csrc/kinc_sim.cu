@@ -579,7 +579,7 @@ extern "C" void kinc_sim_destroy(kinc_sim_ctx* ctx)
    delete ctx;
 }
 
-/* per warp slot scratch of the K-means task pool (kinc::kmeans_pool) */
+/* per warp slot scratch of K-means with a stream of pairs (kinc::k_kmeans_pairs) */
 struct KmPool
 {
    int dmax = 0, tmax = 0, rs = 0;
@@ -599,6 +599,12 @@ static KmPool km_pool_sizes(const kinc_sim_params& p, const SimKernel& k)
 }
 
 /* ---------------------------------------------------------- launch shape */
+
+/* dynamic shared memory of a warp: the sort buffer, and at other times the K-means kernel's ring */
+static size_t warp_smem(const SimKernel& k, size_t sort_bytes)
+{
+   return k.clus == 2 && k.ks > 0 ? std::max(sort_bytes, (size_t)KM_RING_BYTES) : sort_bytes;
+}
 
 /* the shape measured best on the clustering workloads: CTAs of the kernel's full warp count (20
  * for GMM, 16 otherwise), rounds for GMM and no clustering, free-running warps for K-means, the
@@ -740,7 +746,9 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
                                       ? (size_t)7 * ctx->kern.ks * TILE * sizeof(float) : 0;
    const int wpb = ctx->kern.wpb;
    ctx->smem_sort = need_sort && param_bytes_warp == 0 && sort_bytes_warp * wpb <= 200 * 1024;
-   ctx->smem_bytes = (int)((ctx->smem_sort ? sort_bytes_warp : 0) + param_bytes_warp) * wpb;
+   ctx->smem_warp = (int)(warp_smem(ctx->kern, ctx->smem_sort ? sort_bytes_warp : 0) + param_bytes_warp);
+   dp.smem_floats = ctx->smem_warp / (int)sizeof(float);
+   ctx->smem_bytes = ctx->smem_warp * wpb;
    /* opt in whenever dynamic shared memory is used: the kernel's own static words count against 48 KB too */
    if ( ctx->smem_bytes > 0 )
       CKC(cudaFuncSetAttribute(ctx->kern.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->smem_bytes));
@@ -784,7 +792,6 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
    }
    snprintf(ctx->gpu_name, sizeof ctx->gpu_name, "%s", prop.name);
    ctx->slots = (int64_t)slots;
-   ctx->smem_warp = (int)((ctx->smem_sort ? sort_bytes_warp : 0) + param_bytes_warp);
    if ( ctx->gmm_per_sm > 0 )
    {
       CKC(cudaMalloc(&ctx->d_pairs, sim_gmm_pairs_scratch(ctx->sms, dp, ctx->n_cap, nullptr, ctx->dsp)));
@@ -1584,7 +1591,9 @@ extern "C" int kinc_sim_execute_block_noalloc(const float* d_gem, int32_t genes,
    dp.km_dmax = km.dmax;
    dp.km_tmax = km.tmax;
    const int smem_sort = need_sort && param_bytes_warp == 0 && sort_bytes_warp * wpb <= 200 * 1024;
-   const int smem_bytes = (int)((smem_sort ? sort_bytes_warp : 0) + param_bytes_warp) * wpb;
+   const int smem_warp = (int)(warp_smem(kern, smem_sort ? sort_bytes_warp : 0) + param_bytes_warp);
+   dp.smem_floats = smem_warp / (int)sizeof(float);
+   const int smem_bytes = smem_warp * wpb;
    if ( smem_bytes > 0 )
       CK(cudaFuncSetAttribute(kern.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
 

@@ -121,8 +121,9 @@ struct DevParams
    /* launch shape (results are the same for every choice) */
    int32_t warps;                   /* warps per CTA */
    int32_t rounds;                  /* 1: a CTA's warps take their tiles together, round by round */
+   int32_t smem_floats;             /* dynamic shared memory of a warp: its sort buffer or K-means ring */
    int32_t prefetch;                /* samples ahead the EM sweeps prefetch into L2 (0: none) */
-   int32_t km_dmax, km_tmax;        /* K-means task pool: draws per pair, tasks per tile */
+   int32_t km_dmax, km_tmax;        /* K-means: draws per pair, run records per warp */
    float neg_zero;                  /* -0.0f, a value the compiler cannot see (kinc_f2.h: mulz) */
 };
 
@@ -148,8 +149,8 @@ struct DevScratch
    uint32_t* rng;                   /* per warp slot: [31][32] */
    float* sortbuf;                  /* per warp slot: sort_floats, used when not in shared memory */
    float2* Xl;                      /* K-means: per lane [S], the lane's samples contiguous */
-   int32_t* kmd;                    /* K-means task pool: per warp slot [km_dmax][32] rand() draws */
-   float* kmr;                      /* K-means task pool: per warp slot [km_tmax][record floats] */
+   int32_t* kmd;                    /* K-means: per warp slot and open pair, rand() draws */
+   float* kmr;                      /* K-means: per warp slot, records of the open pairs' runs */
 };
 
 struct DevBlock
@@ -168,6 +169,26 @@ struct DevBlock
    unsigned long long* work;        /* [0] model units: sum over fits of iterations x N x K;
                                        [1] fits run */
 };
+
+/* ---------------------------- K-means with a stream of pairs (sim_kmeans_pairs.cuh) */
+
+constexpr int KM_COLS = 8;          /* pairs a warp keeps open */
+constexpr int KM_STAGE = 16;        /* samples of them per stage of the warp's shared-memory ring */
+constexpr int KM_DEPTH = 3;         /* stages */
+constexpr int KM_RING_BYTES = KM_DEPTH * KM_STAGE * KM_COLS * (int)sizeof(float2);   /* of one warp */
+
+/* floats per run's record: assignment means (2K), final means (2K), log-likelihood */
+template <int KT>
+__host__ __device__ constexpr int km_record_floats()
+{
+   return 4 * KT + 1;
+}
+
+/* draws of one pair for K = kmin..kmax (10 initialisations x K each) */
+__host__ __device__ inline int km_draws_per_pair(int kmin, int kmax)
+{
+   return 10 * (kmax * (kmax + 1) / 2 - (kmin - 1) * kmin / 2);
+}
 
 /* ------------------------------------------------------------- helpers */
 

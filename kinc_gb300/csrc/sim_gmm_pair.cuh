@@ -30,7 +30,7 @@
  */
 #pragma once
 
-#include "sim_kernel.cuh"
+#include "sim_pair.cuh"
 
 #include <type_traits>
 
@@ -110,6 +110,13 @@ __device__ __forceinline__ float2 gp_x(const GpView& s, int i)
    const float* q = s.x + (i >> 1) * 4 + (i & 1);
    return make_float2(q[0], q[2]);
 }
+
+/* the samples as the outlier and correlation passes read them */
+struct GpSamples
+{
+   GpView s;
+   __device__ __forceinline__ float2 operator()(int i) const { return gp_x(s, i); }
+};
 
 __device__ __forceinline__ F2 gp_ld2(const float* p)
 {
@@ -791,46 +798,14 @@ __device__ __noinline__ GpFit gp_fit(GpLayout lay, double c2, bool ocl, bool icl
 __device__ inline int gp_fetch(const DevParams& P, const DevData& D, int32_t x, int32_t y, const GpView& s,
                                int8_t* lbl, int lane, bool& xsafe)
 {
-   const float* g1 = D.gem + (size_t)x * P.S;
-   const float* g2 = D.gem + (size_t)y * P.S;
-   constexpr int CH = 4;
-   int n = 0;
    bool fine = true;
-   for ( int base = 0; base < P.S; base += CH * 32 )
-   {
-      float v1[CH], v2[CH];
-#pragma unroll
-      for ( int u = 0; u < CH; ++u )
-      {
-         const int i = base + u * 32 + lane;
-         v1[u] = i < P.S ? __ldg(g1 + i) : 0.f;
-         v2[u] = i < P.S ? __ldg(g2 + i) : 0.f;
-      }
-#pragma unroll
-      for ( int u = 0; u < CH; ++u )
-      {
-         const int i = base + u * 32 + lane;
-         bool use = false;
-         if ( i < P.S )
-         {
-            const bool nanb = isnan(v1[u]) || isnan(v2[u]);
-            const bool low = v1[u] < P.min_expr || v2[u] < P.min_expr;
-            lbl[i] = nanb ? (int8_t)-9 : (low ? (int8_t)-6 : (int8_t)0);
-            use = !nanb && !low;
-         }
-         const unsigned bal = __ballot_sync(0xffffffffu, use);
-         const int at = n + __popc(bal & lanemask_lt());
-         if ( use && at < s.n64 )
-         {
-            float* q = s.x + (at >> 1) * 4 + (at & 1);
-            q[0] = v1[u];
-            q[2] = v2[u];
-            fine = fine && fabsf(v1[u]) <= 1e8f && fabsf(v2[u]) <= 1e8f;
-         }
-         n += __popc(bal);
-      }
-   }
-   __syncwarp();
+   const int n = pair_fetch(P, D, x, y, lbl, lane, [&](int at, float v0, float v1) {
+      if ( at >= s.n64 ) return;
+      float* q = s.x + (at >> 1) * 4 + (at & 1);
+      q[0] = v0;
+      q[2] = v1;
+      fine = fine && fabsf(v0) <= 1e8f && fabsf(v1) <= 1e8f;
+   });
    if ( n > 0 && n <= s.n64 )
    {
       const float2 first = gp_x(s, 0);
@@ -845,184 +820,6 @@ __device__ inline int gp_fetch(const DevParams& P, const DevData& D, int32_t x, 
    xsafe = __all_sync(0xffffffffu, fine);
    __syncwarp();
    return n;
-}
-
-/* Clustering::markOutliers (as warp_mark_outliers) on the pair's arrays */
-__device__ inline void gp_mark_outliers(const GpView& s, int col, int8_t* lbl, int8_t cluster, int8_t marker, int lane)
-{
-   float* buf = s.work;
-   int n = 0;
-   for ( int base = 0; base < s.N; base += 32 )
-   {
-      const int i = base + lane;
-      bool sel = false;
-      if ( i < s.N )
-      {
-         const int8_t l = lbl[i];
-         sel = l == cluster || l == marker;
-      }
-      const unsigned bal = __ballot_sync(0xffffffffu, sel);
-      if ( sel )
-      {
-         const float2 xv = gp_x(s, i);
-         buf[n + __popc(bal & lanemask_lt())] = col == 0 ? xv.x : xv.y;
-      }
-      n += __popc(bal);
-   }
-   if ( n == 0 )
-   {
-      __syncwarp();
-      return;
-   }
-   const int np2 = next_pow2(n);
-   for ( int i = n + lane; i < np2; i += 32 ) buf[i] = __int_as_float(0x7f800000);
-   __syncwarp();
-   warp_bitonic(np2, buf, nullptr, lane);
-   const float Q1 = buf[n * 1 / 4];
-   const float Q3 = buf[n * 3 / 4];
-   const float T_min = Q1 - 1.5f * (Q3 - Q1);
-   const float T_max = Q3 + 1.5f * (Q3 - Q1);
-   for ( int i = lane; i < s.N; i += 32 )
-   {
-      if ( lbl[i] == cluster )
-      {
-         const float2 xv = gp_x(s, i);
-         const float v = col == 0 ? xv.x : xv.y;
-         if ( v < T_min || T_max < v ) lbl[i] = marker;
-      }
-   }
-   __syncwarp();
-}
-
-/* Spearman::computeCluster (as warp_spearman) on the pair's arrays */
-__device__ inline float gp_spearman(const DevParams& P, const DevData& D, const GpView& s, const int8_t* lbl,
-                                    int32_t x, int32_t y, int8_t k, int lane)
-{
-   const int p2 = next_pow2(s.N);
-   float* sx = s.work;
-   float* sy = sx + p2;
-   float* sr = sx;             /* the ranks by x, once the values of x have been sorted */
-   const float* g1 = D.gem + (size_t)x * P.S;
-   const float* g2 = D.gem + (size_t)y * P.S;
-   int n = 0;
-   int jw = 0;
-   for ( int base = 0; base < P.S; base += 32 )
-   {
-      const int i = base + lane;
-      const int8_t l = i < P.S ? lbl[i] : (int8_t)-1;
-      const bool incl = l == k;
-      const unsigned bn = __ballot_sync(0xffffffffu, l >= 0);
-      const unsigned bi = __ballot_sync(0xffffffffu, incl);
-      if ( incl )
-      {
-         const int slot = n + __popc(bi & lanemask_lt());
-         const float2 v = P.semantics == 0 ? gp_x(s, jw + __popc(bn & lanemask_lt())) : make_float2(g1[i], g2[i]);
-         sx[slot] = v.x;
-         sy[slot] = v.y;
-      }
-      n += __popc(bi);
-      jw += __popc(bn);
-   }
-   if ( n < P.min_samples )
-   {
-      __syncwarp();
-      return __int_as_float(0x7fc00000);
-   }
-   const int np2 = next_pow2(n);
-   for ( int i = n + lane; i < np2; i += 32 )
-   {
-      sx[i] = __int_as_float(0x7f800000);
-      sy[i] = __int_as_float(0x7f800000);
-   }
-   __syncwarp();
-   warp_bitonic(np2, sx, sy, lane);
-   for ( int i = lane; i < np2; i += 32 ) sr[i] = i < n ? (float)(i + 1) : 0.f;
-   __syncwarp();
-   warp_bitonic(np2, sy, sr, lane);
-   uint32_t diff = 0;
-   for ( int i = lane; i < n; i += 32 )
-   {
-      const int tmp = (int)((float)(i + 1) - sr[i]);
-      diff += (uint32_t)(tmp * tmp);
-   }
-   for ( int o = 16; o > 0; o >>= 1 ) diff += __shfl_xor_sync(0xffffffffu, diff, o);
-   __syncwarp();
-   const int32_t denom = (int32_t)((uint32_t)n * ((uint32_t)n * (uint32_t)n - 1u));
-   return (float)(1.0 - 6.0 * (double)(int32_t)diff / (double)denom);
-}
-
-/* Pearson::computeCluster (as lane_pearson) of every cluster k < K <= 5: lane 5k + q sums the q-th of
- * cluster k's five sums, in sample position order; lane k returns cluster k's correlation */
-__device__ inline float gp_pearson(const DevParams& P, const DevData& D, const DevBlock& B, const GpView& s,
-                                   const int8_t* lbl, int64_t p, int32_t x, int32_t y, int lane)
-{
-   const int k = lane / 5, q = lane % 5;
-   float acc = 0.f;
-   int n = 0;
-   /* the points of up to 32 consecutive positions, one per lane, added in order */
-   auto add = [&](float vx, float vy, int l, int cnt) {
-      for ( int j = 0; j < cnt; ++j )
-      {
-         const float ax = __shfl_sync(0xffffffffu, vx, j);
-         const float ay = __shfl_sync(0xffffffffu, vy, j);
-         const int al = __shfl_sync(0xffffffffu, l, j);
-         const float a = q == 1 || q == 3 ? ay : ax;
-         const float b = q < 2 ? 1.0f : q == 2 ? ax : ay;
-         if ( al == k )
-         {
-            acc += a * b;
-            ++n;
-         }
-      }
-   };
-   if ( P.semantics == 0 )
-   {
-      for ( int base = 0; base < s.N; base += 32 )
-      {
-         const int i = base + lane;
-         const float2 v = i < s.N ? gp_x(s, i) : make_float2(0.f, 0.f);
-         add(v.x, v.y, i < s.N ? lbl[i] : -1, min(32, s.N - base));
-      }
-      /* positions i >= N: what the last earlier pair of the work block with more than i usable
-       * samples left there (links point strictly backwards, as in lane_pearson) */
-      const int32_t self = (int32_t)(p - B.lo);
-      for ( int base = s.N; base < P.S; base += 32 )
-      {
-         const int i = base + lane;
-         const int l = i < P.S ? lbl[i] : -1;
-         float2 v = make_float2(0.f, 0.f);
-         if ( l >= 0 )
-         {
-            int32_t c = B.pg[self];
-            if ( c >= self ) c = -1;
-            while ( c >= 0 && B.N[c] <= i )
-            {
-               const int32_t nxt = B.pg[c];
-               c = nxt < c ? nxt : -1;
-            }
-            PackedCursor cur;
-            if ( c >= 0 ) v = cur.at(P, D, B.lo + c, i);
-         }
-         __syncwarp();
-         add(v.x, v.y, l, min(32, P.S - base));
-      }
-   }
-   else
-   {
-      const float* g1 = D.gem + (size_t)x * P.S;
-      const float* g2 = D.gem + (size_t)y * P.S;
-      for ( int base = 0; base < P.S; base += 32 )
-      {
-         const int i = base + lane;
-         const bool in = i < P.S;
-         add(in ? g1[i] : 0.f, in ? g2[i] : 0.f, in ? lbl[i] : -1, min(32, P.S - base));
-      }
-   }
-   const int from = lane < GP_KMAX ? 5 * lane : 0;
-   const float sx = __shfl_sync(0xffffffffu, acc, from), sy = __shfl_sync(0xffffffffu, acc, from + 1);
-   const float sxx = __shfl_sync(0xffffffffu, acc, from + 2), syy = __shfl_sync(0xffffffffu, acc, from + 3);
-   const float sxy = __shfl_sync(0xffffffffu, acc, from + 4);
-   return pearson_value(P, __shfl_sync(0xffffffffu, n, from), sx, sy, sxx, syy, sxy);
 }
 
 /* the CTA's active warps wait for one another */
@@ -1093,8 +890,8 @@ k_gmm_pairs(DevParams P, DevData D, DevScratch W, DevBlock B, int smem_floats, i
          s.nch = (n + GP_CHUNK - 1) / GP_CHUNK;
          if ( P.pre_out )
          {
-            gp_mark_outliers(s, 0, lbl, 0, -7, lane);
-            gp_mark_outliers(s, 1, lbl, 0, -7, lane);
+            pair_mark_outliers(GpSamples { s }, n, s.work, 0, lbl, 0, -7, lane);
+            pair_mark_outliers(GpSamples { s }, n, s.work, 1, lbl, 0, -7, lane);
          }
          fits = n >= P.min_samples;
          rng.mode = P.rand_mode;
@@ -1164,31 +961,7 @@ k_gmm_pairs(DevParams P, DevData D, DevScratch W, DevBlock B, int smem_floats, i
             atomicAdd(&B.work[0], units);
             atomicAdd(&B.work[1], (unsigned long long)(P.max_k - P.min_k + 1));
          }
-         if ( P.post_out && K > 1 )
-         {
-            for ( int k = 0; k < K; ++k )
-            {
-               gp_mark_outliers(s, 0, lbl, (int8_t)k, -8, lane);
-               gp_mark_outliers(s, 1, lbl, (int8_t)k, -8, lane);
-            }
-         }
-         const int nc = P.ncorr;
-         float* row = B.outCorr ? B.outCorr + (p - B.start) * P.max_k * nc : nullptr;
-         const float nan = __int_as_float(0x7fc00000);
-         if ( P.corr != 1 && row )
-         {
-            const float r = K > 0 ? gp_pearson(P, D, B, s, lbl, p, x, y, lane) : nan;
-            if ( lane < P.max_k ) row[lane * nc] = lane < K ? r : nan;
-         }
-         if ( P.corr != 0 && row )
-         {
-            for ( int k = 0; k < P.max_k; ++k )
-            {
-               const float r = k < K ? gp_spearman(P, D, s, lbl, x, y, (int8_t)k, lane) : nan;
-               if ( lane == 0 ) row[k * nc + (P.corr == 2 ? 1 : 0)] = r;
-            }
-         }
-         if ( lane == 0 && B.outK ) B.outK[p - B.start] = (int8_t)K;
+         pair_finish(P, D, B, GpSamples { s }, s.work, lbl, p, n, K, lane);
       }
 
       gp_cta_sync(warps);

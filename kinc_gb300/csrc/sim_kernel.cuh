@@ -1,7 +1,8 @@
 /*
  * sim_kernel.cuh -- the per-pair Similarity kernel, specialised by
  * clustering method (CLUS: 0 none, 1 GMM, 2 K-means, 3 GMM as KINC's OpenCL
- * kernels compute it, for rand_mode 1) and by the largest
+ * kernels compute it, for rand_mode 1; K-means up to 5 clusters runs in
+ * sim_kmeans_pairs.cuh instead) and by the largest
  * cluster count compiled with static register arrays (KS = 3 or 5: every
  * fit, whatever its K <= KS, runs the same code with its per-component state
  * in registers, the host picks KS >= maxclus; KS = 0: the generic
@@ -260,12 +261,6 @@ __device__ int lane_cluster(const DevParams& P, const DevData& D, const float2* 
    return bestK;
 }
 
-} /* namespace kinc */
-
-#include "sim_kmeans_pool.cuh"
-
-namespace kinc {
-
 template <int CLUS, int KS>
 __global__ void __launch_bounds__(kernel_warps<CLUS>() * 32, kernel_min_blocks<CLUS>())
 k_similarity(DevParams P, DevData D, DevScratch W, DevBlock B, int smem_sort)
@@ -287,7 +282,7 @@ k_similarity(DevParams P, DevData D, DevScratch W, DevBlock B, int smem_sort)
    int8_t* yb = W.yb + slot * col;
    int8_t* yc = W.yc + slot * col;
    uint32_t* ring = W.rng + slot * (size_t)(RNG_WORDS * TILE);
-   float* sbuf = smem_sort ? smem + (size_t)warp * P.sort_floats : W.sortbuf + slot * (size_t)P.sort_floats;
+   float* sbuf = smem_sort ? smem + (size_t)warp * P.smem_floats : W.sortbuf + slot * (size_t)P.sort_floats;
    /* GMM parameters in shared memory (KINC_GMM_PARAMS_SMEM): 7 arrays of KS x 32 floats per warp */
    float* pbuf = (CM == 1 && KINC_GMM_PARAMS_SMEM && KS > 0)
                     ? smem + (smem_sort ? (size_t)nwarps * P.sort_floats : 0) + (size_t)warp * 7 * KS * TILE
@@ -356,20 +351,7 @@ k_similarity(DevParams P, DevData D, DevScratch W, DevBlock B, int smem_sort)
       {
          unsigned long long units = 0, fits = 0;
          K = 0;
-         if constexpr ( CLUS == 2 && KS > 0 )
-         {
-            /* the tile's runs as one pool of tasks, every lane busy until it is empty */
-            LaneRng rng;
-            rng.ring = ring + lane;
-            rng.head = 0;
-            rng.mode = P.rand_mode;
-            rng.lcg = 1;
-            constexpr int RS = km_record_floats<KS>();
-            K = kmeans_pool<KS>(P, D, X, lbl, ya + lane, yb + lane, wl + lane, lpx + lane,
-                                W.kmd + (size_t)slot * P.km_dmax * TILE, W.kmr + (size_t)slot * P.km_tmax * RS,
-                                npairs, myN, rng, lane, units, fits);
-         }
-         else if ( lane < npairs )
+         if ( lane < npairs )
          {
             LaneRng rng;
             rng.ring = ring + lane;
