@@ -9,7 +9,7 @@
  *   k_scan_*    exclusive prefix of "N >= minsamp" -> each pair's position on
  *               the rand() stream (a serial KINC process draws rand() only for
  *               pairs that reach the clustering loop)
- *   k_prev      previous pair with a larger N inside the same 32768-pair work
+ *   k_links     previous pair with a larger N inside the same 32768-pair work
  *               block (what the reference's stale packed-array reads see)
  *   k_similarity  the per-pair work (sim_device.cuh)
  * Replaces Similarity::OpenCL::{initialize, Worker::Worker, Worker::execute}
@@ -99,14 +99,20 @@ __device__ __forceinline__ int pair_count(const uint32_t* __restrict__ umask, in
    return n;
 }
 
-/* N for pairs [lo, lo + count) */
+/* N for pairs [lo, lo + count), and the largest of every 32 of them (most32 may be NULL) */
 __global__ void k_count(const uint32_t* __restrict__ umask, int W, int64_t lo, int64_t count,
-                        int32_t* __restrict__ N)
+                        int32_t* __restrict__ N, int32_t* __restrict__ most32)
 {
-   for ( int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < count;
-         t += (int64_t)gridDim.x * blockDim.x )
+   const int64_t end = (count + 31) / 32 * 32;      /* whole warps */
+   for ( int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < end; t += (int64_t)gridDim.x * blockDim.x )
    {
-      N[t] = pair_count(umask, W, lo + t);
+      const int n = t < count ? pair_count(umask, W, lo + t) : -1;
+      if ( t < count ) N[t] = n;
+      if ( most32 )
+      {
+         const int m = __reduce_max_sync(0xffffffffu, n);
+         if ( (threadIdx.x & 31) == 0 ) most32[t / 32] = m;
+      }
    }
 }
 
@@ -200,67 +206,84 @@ __global__ void k_scan_apply(const int32_t* __restrict__ N, int64_t offset, int6
    if ( t < count ) qpos[t] = boff[blockIdx.x] + ex;
 }
 
-/* previous pair (same 32768-pair work block) with a strictly larger N: a CTA
- * builds a max-tree of its work block's N in shared memory (internal
- * nodes 1..WB-1; leaf i is N of the block's i-th pair, -1 past its end) and
- * every pair searches it independently -- up the tree until a left sibling
- * holds a larger maximum, then down that subtree keeping to the right.  Links
- * are offsets from lo (-1 = none); lo is a work-block boundary. */
-constexpr int PREV_THREADS = 1024;
-constexpr int PREV_SMEM = KINC_SIM_WORK_BLOCK_SIZE * (int)sizeof(int32_t);
+/*
+ * Links: the previous pair of the same 32768-pair work block with a strictly larger N, as an offset from lo
+ * (-1: none); lo is a work-block boundary.  A CTA answers LINK_GROUP consecutive pairs.  Most find theirs among
+ * the pairs before them in the warp; the others look through the maxima of 32 pairs (left by k_count) back to
+ * the group's start, through those of whole groups, and then down again.  (A max-tree of the whole work block per
+ * CTA took 30 us for 499,500 pairs.)
+ */
+constexpr int LINK_GROUP = 1024;
 
-__global__ void __launch_bounds__(PREV_THREADS) k_prev(const int32_t* __restrict__ N, int64_t lo, int64_t end,
-                                                       int32_t* __restrict__ pg, int split)
+__global__ void __launch_bounds__(LINK_GROUP) k_links(const int32_t* __restrict__ N, const int32_t* __restrict__ most32,
+                                                      int64_t count, int32_t* __restrict__ pg)
 {
-   constexpr int WB = KINC_SIM_WORK_BLOCK_SIZE;
-   extern __shared__ int32_t tree[];
-   /* `split` CTAs per work block: each builds the block's tree and answers its share of the pairs */
-   const int part = (int)(blockIdx.x % split);
-   const int64_t b0 = lo + (int64_t)(blockIdx.x / split) * WB;
-   const int64_t n64 = end - b0 < WB ? end - b0 : WB;
-   const int n = (int)n64;
-   const int32_t* Nb = N + (b0 - lo);
-   auto leaf = [&](int i) -> int32_t { return i < n ? Nb[i] : -1; };
-   auto node = [&](int k) -> int32_t { return k >= WB ? leaf(k - WB) : tree[k]; };
-
-   for ( int k = WB / 2 + threadIdx.x; k < WB; k += PREV_THREADS )
-      tree[k] = max(leaf(2 * k - WB), leaf(2 * k + 1 - WB));
+   constexpr int CHUNKS = KINC_SIM_WORK_BLOCK_SIZE / 32, GROUPS = KINC_SIM_WORK_BLOCK_SIZE / LINK_GROUP;
+   __shared__ int32_t chunk[CHUNKS], group[GROUPS];
+   const int lane = threadIdx.x & 31;
+   const int64_t t = blockIdx.x * (int64_t)LINK_GROUP + threadIdx.x;
+   const int64_t block0 = t / KINC_SIM_WORK_BLOCK_SIZE * KINC_SIM_WORK_BLOCK_SIZE;   /* the same for the CTA */
+   const int mine = (int)((blockIdx.x * (int64_t)LINK_GROUP - block0) / LINK_GROUP);
+   /* maxima of this group's and the earlier groups' chunks */
+   for ( int i = threadIdx.x; i < (mine + 1) * 32; i += LINK_GROUP )
+   {
+      const int64_t c = block0 / 32 + i;
+      chunk[i] = c * 32 < count ? most32[c] : -1;
+   }
    __syncthreads();
-   for ( int level = WB / 4; level >= 1; level >>= 1 )
+   if ( (threadIdx.x >> 5) < mine )
    {
-      for ( int k = level + threadIdx.x; k < 2 * level; k += PREV_THREADS ) tree[k] = max(tree[2 * k], tree[2 * k + 1]);
-      __syncthreads();
+      const int m = __reduce_max_sync(0xffffffffu, chunk[threadIdx.x]);
+      if ( lane == 0 ) group[threadIdx.x >> 5] = m;
    }
-   const int share = (n + split - 1) / split;
-   const int o_end = min(n, (part + 1) * share);
-   for ( int o = part * share + threadIdx.x; o < o_end; o += PREV_THREADS )
+   __syncthreads();
+   const int v = t < count ? N[t] : 0x7fffffff;
+   /* in the warp: m[k] is the largest of the 2^k pairs up to this lane; from the widest down, whole stretches
+    * without a larger N are stepped over */
+   int m[5];
+   m[0] = v;
+#pragma unroll
+   for ( int k = 1; k < 5; ++k )
    {
-      const int32_t v = Nb[o];
-      int ans = -1;
-      for ( int idx = WB + o; idx > 1; idx >>= 1 )
+      const int up = __shfl_up_sync(0xffffffffu, m[k - 1], 1 << (k - 1));
+      m[k] = lane >= 1 << (k - 1) ? max(m[k - 1], up) : m[k - 1];
+   }
+   int from = lane - 1;
+#pragma unroll
+   for ( int k = 4; k >= 0; --k )
+   {
+      const int most = __shfl_sync(0xffffffffu, m[k], max(from, 0));
+      if ( from >= 0 && most <= v ) from -= 1 << k;
+   }
+   /* (a lane past the stretch's start covers fewer pairs; below zero there is none) */
+   if ( t >= count ) return;
+   if ( from >= 0 )
+   {
+      pg[t] = (int32_t)(t - lane + from);
+      return;
+   }
+   int c = mine * 32 + (threadIdx.x >> 5) - 1;
+   while ( c >= mine * 32 && chunk[c] <= v ) --c;
+   if ( c < mine * 32 )
+   {
+      int g = mine - 1;
+      while ( g >= 0 && group[g] <= v ) --g;
+      if ( g < 0 )
       {
-         if ( !(idx & 1) || node(idx - 1) <= v ) continue;
-         int s = idx - 1;            /* the nearest range to the left with a larger N */
-         while ( s < WB ) s = node(2 * s + 1) > v ? 2 * s + 1 : 2 * s;
-         ans = s - WB;
-         break;
+         pg[t] = -1;
+         return;
       }
-      pg[(b0 - lo) + o] = ans >= 0 ? (int32_t)((b0 - lo) + ans) : -1;
+      c = g * 32 + 31;
+      while ( chunk[c] <= v ) --c;
    }
+   int64_t at = block0 + (int64_t)c * 32 + 31;
+   while ( N[at] <= v ) --at;
+   pg[t] = (int32_t)at;
 }
 
-/* the links of every work block of [lo, end) (lo a work-block boundary) */
-cudaError_t launch_prev(const int32_t* N, int64_t lo, int64_t end, int32_t* pg, cudaStream_t st)
+cudaError_t launch_links(const int32_t* N, const int32_t* most32, int64_t count, int32_t* pg, cudaStream_t st)
 {
-   const cudaError_t attr = cudaFuncSetAttribute(k_prev, cudaFuncAttributeMaxDynamicSharedMemorySize, PREV_SMEM);
-   if ( attr != cudaSuccess ) return attr;
-   const int64_t nwb = (end - 1) / KINC_SIM_WORK_BLOCK_SIZE - lo / KINC_SIM_WORK_BLOCK_SIZE + 1;
-   int dev = 0, sms = 0;
-   cudaGetDevice(&dev);
-   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-   /* enough CTAs for two per SM: a few work blocks split their pairs over several CTAs */
-   const int split = (int)std::max<int64_t>(1, std::min<int64_t>(16, (2 * (int64_t)sms + nwb - 1) / nwb));
-   k_prev<<<(int)(nwb * split), PREV_THREADS, PREV_SMEM, st>>>(N, lo, end, pg, split);
+   k_links<<<(int)((count + LINK_GROUP - 1) / LINK_GROUP), LINK_GROUP, 0, st>>>(N, most32, count, pg);
    return cudaGetLastError();
 }
 
@@ -338,6 +361,7 @@ struct kinc_sim_ctx
    int gmm_per_sm = 0;              /* GMM with one warp per pair (sim_gmm_pair.cuh): pairs an SM holds, 0: not available */
    int64_t gmm_wave = 0;            /* pairs the tile kernel runs at once */
    DevScratch dsp {};               /* its scratch */
+   SpearmanOrders orders {};        /* Spearman without clustering (sim_none.cu); order NULL: the tile kernel */
    kinc_sim_launch launch {};
    char gpu_name[256] = "";
    int64_t max_block = 0;
@@ -349,6 +373,7 @@ struct kinc_sim_ctx
    uint32_t* d_rng0 = nullptr;
    int32_t* d_N = nullptr;
    int32_t* d_pg = nullptr;
+   int32_t* d_most32 = nullptr;
    uint64_t* d_qpos = nullptr;
    unsigned long long* d_bsum = nullptr;
    unsigned long long* d_qbase = nullptr;
@@ -364,6 +389,7 @@ struct kinc_sim_ctx
    float* d_corr = nullptr;
    void* d_scratch = nullptr;
    void* d_pairs = nullptr;
+   void* d_orders = nullptr;
    /* host-side tracking of the rand() position held in d_qbase */
    int64_t q_valid_end = 0;
    int32_t launches = 0;
@@ -563,9 +589,9 @@ extern "C" int kinc_sim_work_counters(kinc_sim_ctx* ctx, uint64_t* out, int rese
 
 static void release(kinc_sim_ctx* c)
 {
-   void* ptrs[] = { c->d_gem, c->d_umask, c->d_logn, c->d_jump, c->d_rng0, c->d_N, c->d_pg, c->d_qpos,
+   void* ptrs[] = { c->d_gem, c->d_umask, c->d_logn, c->d_jump, c->d_rng0, c->d_N, c->d_pg, c->d_most32, c->d_qpos,
                     c->d_bsum, c->d_qbase, c->d_tiles, c->d_work, c->d_compact, c->d_order, c->d_bins, c->d_status, c->d_K, c->d_labels, c->d_corr,
-                    c->d_scratch, c->d_pairs };
+                    c->d_scratch, c->d_pairs, c->d_orders };
    for ( void* p : ptrs )
       if ( p ) cudaFree(p);
    tc_release(c->tc);
@@ -797,8 +823,20 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
       CKC(cudaMalloc(&ctx->d_pairs, sim_gmm_pairs_scratch(ctx->sms, dp, ctx->n_cap, nullptr, ctx->dsp)));
       sim_gmm_pairs_scratch(ctx->sms, dp, ctx->n_cap, (char*)ctx->d_pairs, ctx->dsp);
    }
-   /* a whole wave is the tile kernel's best case: without one, nothing runs there */
-   if ( !sim_gmm_pairs_better(ctx->gmm_per_sm, ctx->gmm_wave, ctx->gmm_wave) )
+   if ( params->precision == 0 && sim_spearman_orders_fit(dp) )
+   {
+      CKC(cudaMalloc(&ctx->d_orders, sim_spearman_orders_bytes(ctx->sms, dp, nullptr, nullptr)));
+      sim_spearman_orders_bytes(ctx->sms, dp, (char*)ctx->d_orders, &ctx->orders);
+      DevData dd {};
+      dd.gem = ctx->d_gem;
+      dd.umask = ctx->d_umask;
+      CKC(sim_spearman_orders(ctx->stream, dp, dd, ctx->orders));
+   }
+   /* the tile kernel's scratch, where a block may run there (a whole wave is its best case against GMM with one
+    * warp per pair; without clustering it is left with Spearman of more samples than the orders take) */
+   const bool tiles = params->precision == 0 && (params->clus_method != 0 || (params->corr_method != 0 && !ctx->d_orders))
+                      && !sim_gmm_pairs_better(ctx->gmm_per_sm, ctx->gmm_wave, ctx->gmm_wave);
+   if ( tiles )
    {
       size_t off = 0;
       auto take = [&](size_t bytes) {
@@ -846,6 +884,7 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
    const int64_t nscan = (ctx->max_block + SCAN_THREADS - 1) / SCAN_THREADS;
    CKC(cudaMalloc(&ctx->d_N, nspan * sizeof(int32_t)));
    CKC(cudaMalloc(&ctx->d_pg, nspan * sizeof(int32_t)));
+   CKC(cudaMalloc(&ctx->d_most32, (nspan / 32 + 1) * sizeof(int32_t)));
    CKC(cudaMalloc(&ctx->d_qpos, (params->precision != 0 ? 4096 : ctx->max_block) * sizeof(uint64_t)));
    CKC(cudaMalloc(&ctx->d_bsum, (nscan + 1) * sizeof(unsigned long long)));
    CKC(cudaMalloc(&ctx->d_qbase, sizeof(unsigned long long)));
@@ -917,9 +956,13 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
    const int64_t span = end - lo;
    int launches = 0;
 
-   k_count<<<(int)std::min<int64_t>((span + 255) / 256, 65535), 256, 0, st>>>(ctx->d_umask, ctx->W, lo, span,
-                                                                               ctx->d_N);
-   ++launches;
+   const bool orders = ctx->orders.order != nullptr;      /* Spearman from the genes' orders counts by itself */
+   if ( !orders || dp.corr == 2 )
+   {
+      k_count<<<(int)std::min<int64_t>((span + 255) / 256, 65535), 256, 0, st>>>(ctx->d_umask, ctx->W, lo, span,
+                                                                                  ctx->d_N, ctx->d_most32);
+      ++launches;
+   }
    if ( dp.clus != 0 && dp.rand_mode == 0 )
    {
       if ( ctx->q_valid_end != start )
@@ -945,12 +988,12 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
    if ( (dp.corr == 0 || dp.corr == 2) && dp.semantics == 0 )
    {
       /* every Pearson run with the reference's packed-array reads needs the links */
-      CK(launch_prev(ctx->d_N, lo, end, ctx->d_pg, st));
+      CK(launch_links(ctx->d_N, ctx->d_most32, span, ctx->d_pg, st));
       ++launches;
    }
    /* Pearson without clustering runs one thread per pair straight from the matrix (no tiles) */
-   const bool lanes = dp.clus == 0 && dp.corr == 0;
-   if ( ctx->d_order && size > TILE && !lanes )
+   const bool lanes = dp.clus == 0 && (dp.corr == 0 || (dp.corr == 2 && orders));
+   if ( ctx->d_order && size > TILE && !lanes && !orders )
    {
       const int64_t off = start - lo;
       const int g = (int)std::min<int64_t>((size + BIN_THREADS - 1) / BIN_THREADS, 1024);
@@ -977,7 +1020,16 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
    B.work = ctx->d_work;
    if ( lanes )
    {
-      CK(sim_launch_pearson_lanes(ctx->sms, st, dp, ctx->dd, B));
+      CK(sim_launch_pearson(ctx->sms, st, dp, ctx->dd, B));
+      if ( orders )
+      {
+         ++launches;
+         CK(sim_launch_spearman(ctx->sms, st, dp, ctx->dd, B, ctx->orders));
+      }
+   }
+   else if ( orders )
+   {
+      CK(sim_launch_spearman(ctx->sms, st, dp, ctx->dd, B, ctx->orders));
    }
    else if ( sim_gmm_pairs_better(ctx->gmm_per_sm, size, ctx->gmm_wave) )
    {
@@ -1313,7 +1365,7 @@ extern "C" int kinc_sim_pair_counts(kinc_sim_ctx* ctx, int64_t start, int64_t si
    {
       const int64_t n = std::min<int64_t>(ctx->max_block, size - done);
       k_count<<<(int)std::min<int64_t>((n + 255) / 256, 65535), 256, 0, ctx->stream>>>(
-         ctx->d_umask, ctx->W, start + done, n, ctx->d_N);
+         ctx->d_umask, ctx->W, start + done, n, ctx->d_N, nullptr);
       CK(cudaGetLastError());
       CK(cudaMemcpyAsync(out_N + done, ctx->d_N, n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
       CK(cudaStreamSynchronize(ctx->stream));
@@ -1673,7 +1725,8 @@ extern "C" int kinc_sim_execute_block_noalloc(const float* d_gem, int32_t genes,
    CK(cudaMemcpyAsync(d_logn, g_noalloc_host_logn, (size_t)(S + 1) * sizeof(double), cudaMemcpyHostToDevice, st));
    k_masks<<<std::max(1, std::min(65535, (int)(((int64_t)genes * W + 255) / 256))), 256, 0, st>>>(
       d_gem, genes, S, W, params->min_expr, d_umask);
-   k_count<<<(int)std::min<int64_t>((span + 255) / 256, 65535), 256, 0, st>>>(d_umask, W, lo, span, d_N);
+   int32_t* d_most32 = (int32_t*)(base + off);      /* in the warps' scratch, before they use it */
+   k_count<<<(int)std::min<int64_t>((span + 255) / 256, 65535), 256, 0, st>>>(d_umask, W, lo, span, d_N, d_most32);
    if ( dp.clus != 0 && dp.rand_mode == 0 )
    {
       if ( start > 0 )
@@ -1685,7 +1738,7 @@ extern "C" int kinc_sim_execute_block_noalloc(const float* d_gem, int32_t genes,
    }
    if ( (dp.corr == 0 || dp.corr == 2) && dp.semantics == 0 )
    {
-      CK(launch_prev(d_N, lo, end, d_pg, st));
+      CK(launch_links(d_N, d_most32, span, d_pg, st));
    }
    CK(cudaGetLastError());
    DevData dd {};

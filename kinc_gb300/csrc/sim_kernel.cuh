@@ -476,9 +476,6 @@ SimKernel sim_kernel_select(int clus, int max_k);
 cudaError_t sim_kernel_launch_any(const SimKernel& k, int grid, int smem, cudaStream_t st, const DevParams& P,
                                   const DevData& D, const DevScratch& W, const DevBlock& B, int smem_sort);
 SimKernel sim_kernel_none();
-/* Pearson without clustering, one thread per pair (sim_none.cu) */
-cudaError_t sim_launch_pearson_lanes(int sms, cudaStream_t st, const DevParams& P, const DevData& D,
-                                     const DevBlock& B);
 /* GMM with one warp per pair (sim_gmm_pair.cu): pairs an SM holds when no pair has more than n_cap usable
  * samples (0: these arguments do not run there), whether a block of `size` pairs runs faster there than in
  * the tile kernel's waves of `wave` pairs, the scratch (labels and responsibilities of the pairs in
@@ -488,6 +485,22 @@ bool sim_gmm_pairs_better(int per_sm, int64_t size, int64_t wave);
 size_t sim_gmm_pairs_scratch(int sms, const DevParams& P, int n_cap, char* base, DevScratch& W);
 cudaError_t sim_launch_gmm_pairs(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevScratch& W,
                                  const DevBlock& B, int n_cap);
+/* Pearson without clustering (sim_none.cu) */
+cudaError_t sim_launch_pearson(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B);
+/* Spearman without clustering from every gene's sample order (sim_none.cu): whether these arguments run there,
+ * the orders of a matrix (the bytes they and the launches' buffers take, laid out from base; and their kernel),
+ * and the launch */
+struct SpearmanOrders
+{
+   uint16_t* order;                             /* [G][S] */
+   uint8_t* ties;                               /* [G] */
+   float* buf;                                  /* per warp, for pairs with equal values */
+};
+bool sim_spearman_orders_fit(const DevParams& P);
+size_t sim_spearman_orders_bytes(int sms, const DevParams& P, char* base, SpearmanOrders* out);
+cudaError_t sim_spearman_orders(cudaStream_t st, const DevParams& P, const DevData& D, const SpearmanOrders& R);
+cudaError_t sim_launch_spearman(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B,
+                                const SpearmanOrders& R);
 SimKernel sim_kernel_gmm(int max_k, bool opencl);
 SimKernel sim_kernel_kmeans(int max_k);
 cudaError_t sim_launch_none(const SimKernel& k, int grid, int smem, cudaStream_t st, const DevParams& P,

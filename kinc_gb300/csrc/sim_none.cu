@@ -1,7 +1,9 @@
-/* Similarity kernel specialisation without clustering (clusmethod none). */
-#include "sim_kernel.cuh"
+/* Similarity without clustering (clusmethod none): Pearson with one thread per pair, Spearman from every
+ * gene's sample order, and the tile kernel's specialisation for what is left. */
+#include "sim_pair.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace kinc {
 
@@ -23,7 +25,7 @@ cudaError_t sim_launch_none(const SimKernel&, int grid, int smem, cudaStream_t s
  * so Pearson::computeCluster (pairwise_pearson.cpp:12-52) reduces to: for every usable position i,
  * in order, add the point the reference reads there -- semantics 0: its packed array at i, which
  * for i < N is the pair's own i-th usable sample and for i >= N what the last earlier pair of the
- * work block with more than i usable samples left (the k_prev links; zero if none); semantics 1:
+ * work block with more than i usable samples left (the k_links links; zero if none); semantics 1:
  * sample i itself.  Same sums in the same order as lane_pearson, so the same bits.
  */
 __global__ void __launch_bounds__(256) k_pearson_lanes(DevParams P, DevData D, DevBlock B)
@@ -119,11 +121,528 @@ __global__ void __launch_bounds__(256) k_pearson_lanes(DevParams P, DevData D, D
    }
 }
 
-cudaError_t sim_launch_pearson_lanes(int sms, cudaStream_t st, const DevParams& P, const DevData& D,
+static cudaError_t sim_launch_pearson_lanes(int sms, cudaStream_t st, const DevParams& P, const DevData& D,
                                      const DevBlock& B)
 {
    const int64_t blocks = std::min<int64_t>((B.size + 255) / 256, (int64_t)sms * 16);
    k_pearson_lanes<<<(int)std::max<int64_t>(1, blocks), 256, 0, st>>>(P, D, B);
+   return cudaGetLastError();
+}
+
+/*
+ * The same for matrices of up to PT_WORDS * 32 samples, on tiles of 16 x 32 genes: the threads of a CTA
+ * share the tile's values in shared memory, 32 samples at a time and zero where unusable, and each sums four
+ * pairs (2 x 2 genes) in registers.  Which samples a pair adds is a bit mask per 32 samples: the usable ones,
+ * or with semantics 0 those of them whose rank is itself a usable position (the r-th usable sample is read at
+ * position r), so every addition is one predicated instruction.  The points that positions i >= N read follow:
+ * the chain of earlier pairs with larger counts N_c, each giving its last N_c - i usable samples.
+ *
+ * One thread per pair straight from the matrix rows (k_pearson_lanes) issued 49 instructions per sample and
+ * touched 32 rows per load; this one issues 9 to 11 (5 predicated additions, the bit test, the products) and
+ * keeps 0.85 of the issue slots busy.  All pairs of 1,237 x 611 (semantics 1): 633 -> 200 us; of 1,000 x 200
+ * (semantics 0): 375 -> 168 us with the launches before it, 45 % of it the points of earlier pairs.
+ */
+constexpr int PT_THREADS = 128;
+constexpr int PT_WORDS = 128;
+
+/* a tile of TX x (512 / TX) genes; few rows x take flat tiles */
+template <int TX>
+struct PearsonTile
+{
+   static constexpr int X = TX, Y = 4 * PT_THREADS / TX;
+   static constexpr int GENES = X + Y;
+   static constexpr int ROW = GENES + 2;    /* floats between samples */
+   static size_t bytes(int W) { return (size_t)(32 * ROW + GENES * W) * sizeof(float); }
+};
+
+/* bits moved, in order, to the set positions of u */
+__device__ __forceinline__ uint32_t deposit_bits(uint32_t bits, uint32_t u)
+{
+   /* make room at every clear position, from the lowest up */
+   uint32_t clear = ~u;
+   while ( clear )
+   {
+      const uint32_t below = (clear & (0u - clear)) - 1u;
+      bits = (bits & below) | ((bits & ~below) << 1);
+      clear &= clear - 1u;
+   }
+   return bits;
+}
+
+/* the five sums of a pair */
+struct PearsonSums
+{
+   float x = 0.f, y = 0.f, xx = 0.f, yy = 0.f, xy = 0.f;
+};
+
+/* one sample added if bit `b` of `in` is set */
+__device__ __forceinline__ void pearson_add(PearsonSums& s, uint32_t in, int b, float vx, float vy, float vxx, float vyy,
+                                            float vxy)
+{
+   asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tand.b32 t, %5, %6;\n\tsetp.ne.u32 p, t, 0;\n\t"
+       "@p add.rn.f32 %0, %0, %7;\n\t@p add.rn.f32 %1, %1, %8;\n\t@p add.rn.f32 %2, %2, %9;\n\t"
+       "@p add.rn.f32 %3, %3, %10;\n\t@p add.rn.f32 %4, %4, %11;\n\t}"
+       : "+f"(s.x), "+f"(s.y), "+f"(s.xx), "+f"(s.yy), "+f"(s.xy)
+       : "r"(in), "r"(1u << b), "f"(vx), "f"(vy), "f"(vxx), "f"(vyy), "f"(vxy));
+}
+
+/* positions i >= N: what the last earlier pair of the work block with more than i usable samples left there.
+ * Pair p = (x, y) of B.lo's span; mx, my: its genes' masks.  (Slower, for all pairs of 1,000 x 200: one flat loop
+ * over the pair's positions, so that the lanes of a warp advance together, 186 us against 166; four points in
+ * flight, 176 us.) */
+__device__ inline void pearson_stale(const DevParams& P, const DevData& D, const DevBlock& B, int64_t p, int32_t x, int N,
+                                     const uint32_t* mx, const uint32_t* my, PearsonSums& sums)
+{
+   const int32_t self = (int32_t)(p - B.lo);
+   const int64_t row0 = (int64_t)x * (x - 1) / 2;
+   int32_t c = B.pg[self];
+   /* links point strictly backwards; anything else ends the walk */
+   if ( c >= self ) c = -1;
+   int i = N;
+   while ( c >= 0 )
+   {
+      const int Nc = B.N[c];
+      const int32_t next = B.pg[c];
+      const int64_t pc = B.lo + c;
+      int32_t xc = x, yc = (int32_t)(pc - row0);
+      if ( pc < row0 ) pair_xy(pc, xc, yc);
+      const uint32_t* ux = D.umask + (size_t)xc * P.W;
+      const uint32_t* uy = D.umask + (size_t)yc * P.W;
+      const float* g1 = D.gem + (size_t)xc * P.S;
+      const float* g2 = D.gem + (size_t)yc * P.S;
+      /* its samples of rank i..Nc-1 are its last Nc - i: found from the end */
+      int w = P.W - 1, left = Nc - i;
+      uint32_t m = __ldg(ux + w) & __ldg(uy + w);
+      while ( __popc(m) < left && w > 0 )
+      {
+         left -= __popc(m);
+         --w;
+         m = __ldg(ux + w) & __ldg(uy + w);
+      }
+      uint32_t low = m;
+      for ( ; left > 0 && low; --left ) low &= ~(0x80000000u >> __clz((int)low));
+      m &= ~low;
+      for ( ; i < Nc; ++i )
+      {
+         while ( !m && w + 1 < P.W )
+         {
+            ++w;
+            m = __ldg(ux + w) & __ldg(uy + w);
+         }
+         const int s = w * 32 + __ffs((int)m) - 1;
+         m &= m - 1u;
+         if ( ((mx[i >> 5] & my[i >> 5]) >> (i & 31)) & 1u )
+         {
+            const float vx = __ldg(g1 + s), vy = __ldg(g2 + s);
+            sums.x += vx;
+            sums.y += vy;
+            sums.xx += vx * vx;
+            sums.yy += vy * vy;
+            sums.xy += vx * vy;
+         }
+      }
+      c = next < c ? next : -1;
+   }
+   /* beyond the longest of them the array still holds zeros, which change no sum */
+}
+
+template <int TX>
+__global__ void __launch_bounds__(PT_THREADS)
+k_pearson_tiles(DevParams P, DevData D, DevBlock B, int x0)
+{
+   constexpr int PT_X = PearsonTile<TX>::X, PT_Y = PearsonTile<TX>::Y, PT_GENES = PearsonTile<TX>::GENES,
+                 PT_ROW = PearsonTile<TX>::ROW;
+   extern __shared__ __align__(16) float pt_smem[];
+   float* v = pt_smem;                                            /* [32][PT_ROW] */
+   uint32_t* mask = (uint32_t*)(pt_smem + 32 * PT_ROW);           /* [PT_GENES][W] */
+   const int gx = x0 + blockIdx.y * PT_X, gy = blockIdx.x * PT_Y;
+   /* pairs (x, y), x > y, of [start, end): nothing here? */
+   const int xl = min(gx + PT_X - 1, P.G - 1);
+   if ( gy >= xl ) return;
+   {
+      const int64_t first = (int64_t)gx * (gx - 1) / 2 + gy, last = (int64_t)xl * (xl - 1) / 2 + min(gy + PT_Y - 1, xl - 1);
+      if ( last < B.start || first >= B.start + B.size ) return;
+   }
+   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+   const int tx = 2 * (tid / (PT_Y / 2)), ty = 2 * (tid % (PT_Y / 2));
+   auto gene = [&](int i) { return i < PT_X ? gx + i : gy + i - PT_X; };
+   for ( int i = tid; i < PT_GENES * P.W; i += PT_THREADS )
+   {
+      const int g = gene(i / P.W);
+      mask[i] = g < P.G ? __ldg(D.umask + (size_t)g * P.W + i % P.W) : 0u;
+   }
+   /* the next 32 samples of the tile on their way in registers: gene warp + 4k, sample lane */
+   constexpr int PER = (PT_GENES + PT_THREADS / 32 - 1) / (PT_THREADS / 32);
+   float next[PER];
+   auto fetch = [&](int w) {
+      const int s = w * 32 + lane;
+#pragma unroll
+      for ( int k = 0; k < PER; ++k )
+      {
+         const int i = warp + k * (PT_THREADS / 32), g = gene(i);
+         next[k] = i < PT_GENES && g < P.G && s < P.S ? __ldg(D.gem + (size_t)g * P.S + s) : 0.f;
+      }
+   };
+   fetch(0);
+   __syncthreads();
+
+   const uint32_t* mx[2] = { mask + tx * P.W, mask + (tx + 1) * P.W };
+   const uint32_t* my[2] = { mask + (PT_X + ty) * P.W, mask + (PT_X + ty + 1) * P.W };
+   PearsonSums sums[2][2];
+   int n[2][2] = { { 0, 0 }, { 0, 0 } };
+   for ( int w = 0; w < P.W; ++w )
+   {
+#pragma unroll
+      for ( int k = 0; k < PER; ++k )
+      {
+         const int i = warp + k * (PT_THREADS / 32);
+         if ( i < PT_GENES ) v[lane * PT_ROW + i] = (mask[i * P.W + w] >> lane) & 1u ? next[k] : 0.f;
+      }
+      __syncthreads();
+      if ( w + 1 < P.W ) fetch(w + 1);
+      uint32_t in[2][2];
+#pragma unroll
+      for ( int a = 0; a < 2; ++a )
+#pragma unroll
+         for ( int b = 0; b < 2; ++b )
+         {
+            const uint32_t u = mx[a][w] & my[b][w];
+            uint32_t take = u;
+            if ( P.semantics == 0 )
+            {
+               const int r = n[a][b], k = r >> 5, k1 = min(k + 1, P.W - 1);
+               take = deposit_bits(__funnelshift_r(mx[a][k] & my[b][k], mx[a][k1] & my[b][k1], r & 31), u);
+            }
+            in[a][b] = take;
+            n[a][b] += __popc(u);
+         }
+#pragma unroll 8
+      for ( int s = 0; s < 32; ++s )
+      {
+         const float2 vx = *reinterpret_cast<const float2*>(v + s * PT_ROW + tx);
+         const float2 vy = *reinterpret_cast<const float2*>(v + s * PT_ROW + PT_X + ty);
+         const float xs[2] = { vx.x, vx.y }, ys[2] = { vy.x, vy.y };
+         const float xq[2] = { vx.x * vx.x, vx.y * vx.y }, yq[2] = { vy.x * vy.x, vy.y * vy.y };
+#pragma unroll
+         for ( int a = 0; a < 2; ++a )
+#pragma unroll
+            for ( int b = 0; b < 2; ++b ) pearson_add(sums[a][b], in[a][b], s, xs[a], ys[b], xq[a], yq[b], xs[a] * ys[b]);
+      }
+      __syncthreads();
+   }
+#pragma unroll
+   for ( int a = 0; a < 2; ++a )
+#pragma unroll
+      for ( int b = 0; b < 2; ++b )
+      {
+         const int x = gx + tx + a, y = gy + ty + b;
+         if ( x >= P.G || y >= x ) continue;
+         const int64_t p = (int64_t)x * (x - 1) / 2 + y, q = p - B.start;
+         if ( q < 0 || q >= B.size ) continue;
+         PearsonSums t = sums[a][b];
+         if ( P.semantics == 0 && n[a][b] < P.S ) pearson_stale(P, D, B, p, x, n[a][b], mx[a], my[b], t);
+         const float r = pearson_value(P, n[a][b], t.x, t.y, t.xx, t.yy, t.xy);
+         if ( B.outK ) B.outK[q] = 1;
+         if ( B.outCorr )
+         {
+            float* row = B.outCorr + q * P.max_k * P.ncorr;
+            row[0] = r;
+            for ( int k = 1; k < P.max_k * P.ncorr; ++k ) row[k] = __int_as_float(0x7fc00000);
+         }
+      }
+}
+
+template <int TX>
+static cudaError_t launch_pearson_tiles(cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B, int x0,
+                                        int x1)
+{
+   const int smem = (int)PearsonTile<TX>::bytes(P.W);
+   const cudaError_t e = cudaFuncSetAttribute(k_pearson_tiles<TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+   if ( e != cudaSuccess ) return e;
+   const dim3 grid((x1 + PearsonTile<TX>::Y - 1) / PearsonTile<TX>::Y, (x1 - x0) / TX + 1);
+   k_pearson_tiles<TX><<<grid, PT_THREADS, smem, st>>>(P, D, B, x0);
+   return cudaGetLastError();
+}
+
+cudaError_t sim_launch_pearson(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B)
+{
+   /* the rows x of the block */
+   auto row_of = [](int64_t p) {
+      int64_t x = (int64_t)((1.0 + std::sqrt(1.0 + 8.0 * (double)p)) / 2.0);
+      while ( x * (x - 1) / 2 > p ) --x;
+      while ( (x + 1) * x / 2 <= p ) ++x;
+      return (int)x;
+   };
+   const int x0 = row_of(B.start), x1 = row_of(B.start + B.size - 1), rows = x1 - x0 + 1;
+   /* the masks of a tile's genes lie in shared memory beside 32 samples of their values */
+   if ( rows <= 2 && PearsonTile<2>::bytes(P.W) <= 100 * 1024 ) return launch_pearson_tiles<2>(st, P, D, B, x0, x1);
+   if ( rows <= 8 && PearsonTile<4>::bytes(P.W) <= 100 * 1024 ) return launch_pearson_tiles<4>(st, P, D, B, x0, x1);
+   if ( P.W <= PT_WORDS ) return launch_pearson_tiles<16>(st, P, D, B, x0, x1);
+   return sim_launch_pearson_lanes(sms, st, P, D, B);
+}
+
+/*
+ * Spearman without clustering.  Spearman::computeCluster (pairwise_spearman.cpp:27-86) sorts the pair's
+ * usable samples by x, then by y, and sums the squared differences of the two ranks.  The ranks among the
+ * samples that both genes have follow from each gene's own sample order: walked in that order, a sample's
+ * rank is the number of samples before it that the other gene has too.  So every gene is sorted once per
+ * matrix (k_gene_order), and a pair costs two walks of S / 32 warp steps instead of two sorting networks:
+ * 262,144 pairs of 1,000 samples (10 % missing) 32.8 -> 5 to 6 ms, three quarters of it the pairs of the next
+ * paragraph.
+ *
+ * Where two equal values of a gene both take part, their order comes from the network's swaps; the walk
+ * finds such pairs (a flag per sample: equal to the next in order) and gives them to the network.
+ */
+constexpr int ORDER_THREADS = 256;
+constexpr int ORDER_MOST = 8192;            /* samples k_gene_order sorts in shared memory (64 KB of keys) */
+constexpr uint16_t ORDER_TIE = 0x8000;
+constexpr int SPEARMAN_WARPS = 8;
+
+/* order[g][r]: the r-th of gene g's usable samples by value, ORDER_TIE set if the next one is equal; filled up
+ * with samples the gene lacks.  ties[g]: 1 if any is set, 2 added if the gene has +inf, with which the network
+ * fills its buffers up. */
+__global__ void __launch_bounds__(ORDER_THREADS)
+k_gene_order(const float* __restrict__ gem, const uint32_t* __restrict__ umask, int G, int S, int W, int P2,
+             uint16_t* __restrict__ order, uint8_t* __restrict__ ties)
+{
+   extern __shared__ unsigned long long key[];
+   for ( int g = blockIdx.x; g < G; g += gridDim.x )
+   {
+      for ( int i = threadIdx.x; i < P2; i += ORDER_THREADS )
+      {
+         unsigned long long k = ~0ull << 16;
+         if ( i < S && ((umask[(size_t)g * W + (i >> 5)] >> (i & 31)) & 1u) )
+         {
+            const float v = gem[(size_t)g * S + i];
+            const uint32_t b = v == 0.f ? 0u : __float_as_uint(v);
+            k = (unsigned long long)(b & 0x80000000u ? ~b : b | 0x80000000u) << 16;
+         }
+         key[i] = k | (unsigned)i;
+      }
+      __syncthreads();
+      for ( int ob = 2; ob <= P2; ob *= 2 )
+      {
+         for ( int t = ob / 2; t >= 1; t /= 2 )
+         {
+            for ( int i = threadIdx.x; i < P2 / 2; i += ORDER_THREADS )
+            {
+               const int a = (i / t) * 2 * t + i % t, b = a + t;
+               const bool up = !(a & ob);
+               const unsigned long long ka = key[a], kb = key[b];
+               if ( (ka > kb) == up )
+               {
+                  key[a] = kb;
+                  key[b] = ka;
+               }
+            }
+            __syncthreads();
+         }
+      }
+      int any = 0;
+      for ( int i = threadIdx.x; i < S; i += ORDER_THREADS )
+      {
+         const unsigned long long k = key[i] >> 16;
+         const bool usable = k <= 0xffffffffull;
+         const bool tie = usable && i + 1 < S && key[i + 1] >> 16 == k;
+         order[(size_t)g * S + i] = (uint16_t)((key[i] & 0x7fffu) | (tie ? ORDER_TIE : 0));
+         any |= (tie ? 1 : 0) | (k == 0xff800000ull ? 2 : 0);
+      }
+      const int tied = __syncthreads_or(any & 1), inf = __syncthreads_or(any & 2);
+      if ( threadIdx.x == 0 ) ties[g] = (uint8_t)((tied ? 1 : 0) | (inf ? 2 : 0));
+   }
+}
+
+bool sim_spearman_orders_fit(const DevParams& P)
+{
+   return P.clus == 0 && P.corr >= 1 && P.S <= ORDER_MOST;
+}
+
+/* CTAs per SM that get room for the network's buffers */
+static int spearman_ctas(const DevParams& P)
+{
+   const int64_t cta = (int64_t)SPEARMAN_WARPS * 2 * P.P2 * (int)sizeof(float);
+   return (int)std::max<int64_t>(1, std::min<int64_t>(6, 2 * 1024 * 1024 / cta));
+}
+
+size_t sim_spearman_orders_bytes(int sms, const DevParams& P, char* base, SpearmanOrders* out)
+{
+   size_t off = 0;
+   auto take = [&](size_t bytes) {
+      char* p = base + off;
+      off += (bytes + 255) & ~(size_t)255;
+      return p;
+   };
+   uint16_t* order = (uint16_t*)take((size_t)P.G * P.S * sizeof(uint16_t));
+   uint8_t* ties = (uint8_t*)take((size_t)P.G);
+   float* buf = (float*)take((size_t)sms * spearman_ctas(P) * SPEARMAN_WARPS * 2 * P.P2 * sizeof(float));
+   if ( out ) *out = SpearmanOrders { order, ties, buf };
+   return off;
+}
+
+cudaError_t sim_spearman_orders(cudaStream_t st, const DevParams& P, const DevData& D, const SpearmanOrders& R)
+{
+   const int smem = P.P2 * (int)sizeof(unsigned long long);
+   const cudaError_t e = cudaFuncSetAttribute(k_gene_order, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+   if ( e != cudaSuccess ) return e;
+   k_gene_order<<<std::min(P.G, 16384), ORDER_THREADS, smem, st>>>(D.gem, D.umask, P.G, P.S, P.W, P.P2, R.order, R.ties);
+   return cudaGetLastError();
+}
+
+/*
+ * One walk: the samples of `order` that `mask` (shared memory) has, in order; use(sample, rank).  With `check`,
+ * *tied is set when two of them are equal in value.
+ */
+template <bool CHECK, class Use>
+__device__ __forceinline__ int spearman_walk(const uint16_t* __restrict__ order, int S, const uint32_t* mask, int lane,
+                                             bool& tied, Use use)
+{
+   constexpr int U = 4;
+   int n = 0;
+   bool open = false;                       /* the last sample taken is equal to all that followed it so far */
+   for ( int base = 0; base < S; base += 32 * U )
+   {
+      uint32_t o[U];
+#pragma unroll
+      for ( int u = 0; u < U; ++u )
+      {
+         const int i = base + u * 32 + lane;
+         o[u] = i < S ? __ldg(order + i) : 0xffffffffu;
+      }
+#pragma unroll
+      for ( int u = 0; u < U; ++u )
+      {
+         const uint32_t s = o[u] & 0x7fffu;
+         const bool in = o[u] != 0xffffffffu && ((mask[s >> 5] >> (s & 31)) & 1u);
+         const unsigned bal = __ballot_sync(0xffffffffu, in);
+         if ( in ) use((int)s, n + __popc(bal & lanemask_lt()));
+         n += __popc(bal);
+         if ( CHECK )
+         {
+            const unsigned eq = __ballot_sync(0xffffffffu, o[u] != 0xffffffffu && (o[u] & ORDER_TIE));
+            /* the samples equal to this lane's run up to the first that is not flagged */
+            const unsigned rest = ~(eq >> lane);
+            const int len = rest ? __ffs((int)rest) - 1 : 32;      /* flagged in a row from this lane on */
+            const unsigned reach = len >= 31 ? 0xfffffffeu : (2u << len) - 2u;
+            bool t = in && ((bal >> lane) & reach);
+            if ( lane == 0 && open && bal )
+            {
+               const int first = __ffs((int)bal) - 1;
+               t = t || (eq & ((1u << first) - 1u)) == (1u << first) - 1u;
+            }
+            tied = tied || __any_sync(0xffffffffu, t);
+            if ( bal )
+            {
+               const int last = 31 - __clz((int)bal);
+               open = (eq >> last) == (0xffffffffu >> last);
+            }
+            else
+            {
+               open = open && eq == 0xffffffffu;
+            }
+         }
+      }
+   }
+   return n;
+}
+
+__global__ void __launch_bounds__(SPEARMAN_WARPS * 32)
+k_spearman_orders(DevParams P, DevData D, DevBlock B, SpearmanOrders R, int warp_bytes, int per_warp)
+{
+   extern __shared__ __align__(16) unsigned char spearman_smem[];
+   const int lane = threadIdx.x & 31;
+   const int warp = threadIdx.x >> 5;
+   unsigned char* base = spearman_smem + (size_t)warp * warp_bytes;
+   uint32_t* mask = (uint32_t*)base;                                     /* samples that both genes have */
+   uint16_t* ranks = (uint16_t*)(base + ((P.W * 4 + 15) & ~15));         /* by x */
+   float* buf = R.buf + ((size_t)blockIdx.x * SPEARMAN_WARPS + warp) * 2 * P.P2;
+   const int c = P.corr == 2 ? 1 : 0;
+   const float nan = __int_as_float(0x7fc00000);
+   const int64_t step = (int64_t)gridDim.x * SPEARMAN_WARPS * per_warp;
+   for ( int64_t q0 = ((int64_t)blockIdx.x * SPEARMAN_WARPS + warp) * per_warp; q0 < B.size; q0 += step )
+   {
+      int32_t x, y;
+      pair_xy(B.start + q0, x, y);
+      for ( int64_t q = q0; q < min(q0 + per_warp, B.size); ++q )
+      {
+         if ( B.outLabels )
+         {
+            const float* g1 = D.gem + (size_t)x * P.S;
+            const float* g2 = D.gem + (size_t)y * P.S;
+            int8_t* row = B.outLabels + q * (int64_t)P.S;
+            for ( int i = lane; i < P.S; i += 32 )
+            {
+               const float v1 = __ldg(g1 + i), v2 = __ldg(g2 + i);
+               row[i] = isnan(v1) || isnan(v2) ? (int8_t)-9 : v1 < P.min_expr || v2 < P.min_expr ? (int8_t)-6 : (int8_t)0;
+            }
+         }
+         const uint32_t* mx = D.umask + (size_t)x * P.W;
+         const uint32_t* my = D.umask + (size_t)y * P.W;
+         for ( int w = lane; w < P.W; w += 32 ) mask[w] = __ldg(mx + w) & __ldg(my + w);
+         __syncwarp();
+         float r = nan;
+         const int tx = R.ties[x], ty = R.ties[y];
+         bool tied = ((tx | ty) & 2) != 0;
+         int n;
+         auto rank = [&](int s, int i) { ranks[s] = (uint16_t)i; };
+         if ( tx )
+            n = spearman_walk<true>(R.order + (size_t)x * P.S, P.S, mask, lane, tied, rank);
+         else
+            n = spearman_walk<false>(R.order + (size_t)x * P.S, P.S, mask, lane, tied, rank);
+         __syncwarp();
+         if ( n >= P.min_samples )
+         {
+            uint32_t diff = 0;
+            auto add = [&](int s, int i) {
+               const int d = i - (int)ranks[s];
+               diff += (uint32_t)(d * d);
+            };
+            if ( ty )
+               spearman_walk<true>(R.order + (size_t)y * P.S, P.S, mask, lane, tied, add);
+            else
+               spearman_walk<false>(R.order + (size_t)y * P.S, P.S, mask, lane, tied, add);
+            if ( tied )
+               r = spearman_network(D.gem + (size_t)x * P.S, D.gem + (size_t)y * P.S, P.S, mask, buf, lane);
+            else
+               r = spearman_value(__reduce_add_sync(0xffffffffu, diff), n);
+         }
+         __syncwarp();
+         float* row = B.outCorr ? B.outCorr + q * P.max_k * P.ncorr : nullptr;
+         if ( row )
+         {
+            if ( P.ncorr == 1 )
+            {
+               for ( int k = lane; k < P.max_k; k += 32 ) row[k] = k == 0 ? r : nan;
+            }
+            else if ( lane == 0 )
+            {
+               row[c] = r;                  /* the Pearson kernel has filled the rest */
+            }
+         }
+         if ( lane == 0 && B.outK ) B.outK[q] = 1;
+         if ( ++y >= x )
+         {
+            y = 0;
+            ++x;
+         }
+      }
+   }
+}
+
+cudaError_t sim_launch_spearman(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B,
+                                const SpearmanOrders& R)
+{
+   const int bytes = ((P.W * 4 + 15) & ~15) + ((P.S * 2 + 15) & ~15);
+   const int smem = bytes * SPEARMAN_WARPS;
+   cudaError_t e = cudaFuncSetAttribute(k_spearman_orders, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+   int per_sm = 1;
+   if ( e == cudaSuccess )
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spearman_orders, SPEARMAN_WARPS * 32, smem);
+   if ( e != cudaSuccess ) return e;
+   int64_t grid = (int64_t)sms * std::max(1, std::min(per_sm, spearman_ctas(P)));
+   /* neighbouring pairs share x, so a warp takes up to 8 of them -- fewer if the warps would run out */
+   const int per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(8, B.size / (grid * SPEARMAN_WARPS * 4)));
+   grid = std::min(grid, (B.size + SPEARMAN_WARPS * per_warp - 1) / (SPEARMAN_WARPS * per_warp));
+   k_spearman_orders<<<(int)grid, SPEARMAN_WARPS * 32, smem, st>>>(P, D, B, R, bytes, per_warp);
    return cudaGetLastError();
 }
 

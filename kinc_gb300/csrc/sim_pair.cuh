@@ -98,6 +98,62 @@ __device__ inline void pair_mark_outliers(X at, int N, float* buf, int col, int8
    __syncwarp();
 }
 
+/* the closing formula of Spearman::computeCluster (pairwise_spearman.cpp:73-82): the sum of squared rank
+ * differences and n(n^2 - 1) are ints */
+__device__ __forceinline__ float spearman_value(uint32_t diff, int n)
+{
+   const int32_t denom = (int32_t)((uint32_t)n * ((uint32_t)n * (uint32_t)n - 1u));
+   return (float)(1.0 - 6.0 * (double)(int32_t)diff / (double)denom);
+}
+
+/* Spearman of n points by the reference's sorting network (sx, sy: room for next_pow2(n) each); the ranks by x
+ * take the place of the sorted x */
+__device__ inline float spearman_sorted(float* sx, float* sy, int n, int lane)
+{
+   float* sr = sx;
+   const int np2 = next_pow2(n);
+   for ( int i = n + lane; i < np2; i += 32 )
+   {
+      sx[i] = __int_as_float(0x7f800000);
+      sy[i] = __int_as_float(0x7f800000);
+   }
+   __syncwarp();
+   warp_bitonic(np2, sx, sy, lane);
+   for ( int i = lane; i < np2; i += 32 ) sr[i] = i < n ? (float)(i + 1) : 0.f;
+   __syncwarp();
+   warp_bitonic(np2, sy, sr, lane);
+   uint32_t diff = 0;
+   for ( int i = lane; i < n; i += 32 )
+   {
+      const int tmp = (int)((float)(i + 1) - sr[i]);
+      diff += (uint32_t)(tmp * tmp);
+   }
+   diff = __reduce_add_sync(0xffffffffu, diff);
+   __syncwarp();
+   return spearman_value(diff, n);
+}
+
+/* the same for the samples of two rows that `mask` has (buf: room for two sorts of S) */
+__device__ inline float spearman_network(const float* g1, const float* g2, int S, const uint32_t* mask, float* buf, int lane)
+{
+   float* sx = buf;
+   float* sy = buf + next_pow2(S);
+   int n = 0;
+   for ( int base = 0; base < S; base += 32 )
+   {
+      const uint32_t m = mask[base >> 5];
+      const int at = n + __popc(m & lanemask_lt());
+      if ( (m >> lane) & 1u )
+      {
+         sx[at] = g1[base + lane];
+         sy[at] = g2[base + lane];
+      }
+      n += __popc(m);
+   }
+   __syncwarp();
+   return spearman_sorted(sx, sy, n, lane);
+}
+
 /* Spearman::computeCluster (as warp_spearman) */
 template <class X>
 __device__ inline float pair_spearman(const DevParams& P, const DevData& D, X at, int N, float* buf,
@@ -106,7 +162,6 @@ __device__ inline float pair_spearman(const DevParams& P, const DevData& D, X at
    const int p2 = next_pow2(N);
    float* sx = buf;
    float* sy = sx + p2;
-   float* sr = sx;             /* the ranks by x, once the values of x have been sorted */
    const float* g1 = D.gem + (size_t)x * P.S;
    const float* g2 = D.gem + (size_t)y * P.S;
    int n = 0;
@@ -133,27 +188,7 @@ __device__ inline float pair_spearman(const DevParams& P, const DevData& D, X at
       __syncwarp();
       return __int_as_float(0x7fc00000);
    }
-   const int np2 = next_pow2(n);
-   for ( int i = n + lane; i < np2; i += 32 )
-   {
-      sx[i] = __int_as_float(0x7f800000);
-      sy[i] = __int_as_float(0x7f800000);
-   }
-   __syncwarp();
-   warp_bitonic(np2, sx, sy, lane);
-   for ( int i = lane; i < np2; i += 32 ) sr[i] = i < n ? (float)(i + 1) : 0.f;
-   __syncwarp();
-   warp_bitonic(np2, sy, sr, lane);
-   uint32_t diff = 0;
-   for ( int i = lane; i < n; i += 32 )
-   {
-      const int tmp = (int)((float)(i + 1) - sr[i]);
-      diff += (uint32_t)(tmp * tmp);
-   }
-   for ( int o = 16; o > 0; o >>= 1 ) diff += __shfl_xor_sync(0xffffffffu, diff, o);
-   __syncwarp();
-   const int32_t denom = (int32_t)((uint32_t)n * ((uint32_t)n * (uint32_t)n - 1u));
-   return (float)(1.0 - 6.0 * (double)(int32_t)diff / (double)denom);
+   return spearman_sorted(sx, sy, n, lane);
 }
 
 /* Pearson::computeCluster (as lane_pearson) of every cluster k < K <= 5: lane 5k + q sums the q-th of
