@@ -374,6 +374,7 @@ struct kinc_sim_ctx
    int32_t* d_N = nullptr;
    int32_t* d_pg = nullptr;
    int32_t* d_most32 = nullptr;
+   int32_t* d_tied = nullptr;                 /* Spearman without clustering: pairs with equal values */
    uint64_t* d_qpos = nullptr;
    unsigned long long* d_bsum = nullptr;
    unsigned long long* d_qbase = nullptr;
@@ -589,7 +590,7 @@ extern "C" int kinc_sim_work_counters(kinc_sim_ctx* ctx, uint64_t* out, int rese
 
 static void release(kinc_sim_ctx* c)
 {
-   void* ptrs[] = { c->d_gem, c->d_umask, c->d_logn, c->d_jump, c->d_rng0, c->d_N, c->d_pg, c->d_most32, c->d_qpos,
+   void* ptrs[] = { c->d_gem, c->d_umask, c->d_logn, c->d_jump, c->d_rng0, c->d_N, c->d_pg, c->d_most32, c->d_tied, c->d_qpos,
                     c->d_bsum, c->d_qbase, c->d_tiles, c->d_work, c->d_compact, c->d_order, c->d_bins, c->d_status, c->d_K, c->d_labels, c->d_corr,
                     c->d_scratch, c->d_pairs, c->d_orders };
    for ( void* p : ptrs )
@@ -825,8 +826,8 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
    }
    if ( params->precision == 0 && sim_spearman_orders_fit(dp) )
    {
-      CKC(cudaMalloc(&ctx->d_orders, sim_spearman_orders_bytes(ctx->sms, dp, nullptr, nullptr)));
-      sim_spearman_orders_bytes(ctx->sms, dp, (char*)ctx->d_orders, &ctx->orders);
+      CKC(cudaMalloc(&ctx->d_orders, sim_spearman_orders_bytes(dp, nullptr, nullptr)));
+      sim_spearman_orders_bytes(dp, (char*)ctx->d_orders, &ctx->orders);
       DevData dd {};
       dd.gem = ctx->d_gem;
       dd.umask = ctx->d_umask;
@@ -900,6 +901,7 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
       CKC(cudaMalloc(&ctx->d_order, ctx->max_block * sizeof(int32_t)));
       CKC(cudaMalloc(&ctx->d_bins, ctx->nbins * sizeof(unsigned int)));
    }
+   if ( ctx->d_orders ) CKC(cudaMalloc(&ctx->d_tied, ctx->max_block * sizeof(int32_t)));
    CKC(cudaMemsetAsync(ctx->d_work, 0, 4 * sizeof(unsigned long long), ctx->stream));
    CKC(cudaMalloc(&ctx->d_K, ctx->max_block));
    if ( params->precision == 0 ) CKC(cudaMalloc(&ctx->d_labels, (size_t)ctx->max_block * S));
@@ -1023,13 +1025,14 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
       CK(sim_launch_pearson(ctx->sms, st, dp, ctx->dd, B));
       if ( orders )
       {
-         ++launches;
-         CK(sim_launch_spearman(ctx->sms, st, dp, ctx->dd, B, ctx->orders));
+         launches += 2;
+         CK(sim_launch_spearman(ctx->sms, st, dp, ctx->dd, B, ctx->orders, ctx->d_tied));
       }
    }
    else if ( orders )
    {
-      CK(sim_launch_spearman(ctx->sms, st, dp, ctx->dd, B, ctx->orders));
+      ++launches;
+      CK(sim_launch_spearman(ctx->sms, st, dp, ctx->dd, B, ctx->orders, ctx->d_tied));
    }
    else if ( sim_gmm_pairs_better(ctx->gmm_per_sm, size, ctx->gmm_wave) )
    {

@@ -488,19 +488,18 @@ cudaError_t sim_launch_gmm_pairs(int sms, cudaStream_t st, const DevParams& P, c
 /* Pearson without clustering (sim_none.cu) */
 cudaError_t sim_launch_pearson(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B);
 /* Spearman without clustering from every gene's sample order (sim_none.cu): whether these arguments run there,
- * the orders of a matrix (the bytes they and the launches' buffers take, laid out from base; and their kernel),
- * and the launch */
+ * the orders of a matrix (the bytes they take, laid out from base; and their kernel), and the launch
+ * (tied_pairs: room for the block's pairs; B.tiles counts them, zero at first) */
 struct SpearmanOrders
 {
    uint16_t* order;                             /* [G][S] */
    uint8_t* ties;                               /* [G] */
-   float* buf;                                  /* per warp, for pairs with equal values */
 };
 bool sim_spearman_orders_fit(const DevParams& P);
-size_t sim_spearman_orders_bytes(int sms, const DevParams& P, char* base, SpearmanOrders* out);
+size_t sim_spearman_orders_bytes(const DevParams& P, char* base, SpearmanOrders* out);
 cudaError_t sim_spearman_orders(cudaStream_t st, const DevParams& P, const DevData& D, const SpearmanOrders& R);
 cudaError_t sim_launch_spearman(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B,
-                                const SpearmanOrders& R);
+                                const SpearmanOrders& R, int32_t* tied_pairs);
 SimKernel sim_kernel_gmm(int max_k, bool opencl);
 SimKernel sim_kernel_kmeans(int max_k);
 cudaError_t sim_launch_none(const SimKernel& k, int grid, int smem, cudaStream_t st, const DevParams& P,

@@ -387,11 +387,12 @@ cudaError_t sim_launch_pearson(int sms, cudaStream_t st, const DevParams& P, con
  * samples that both genes have follow from each gene's own sample order: walked in that order, a sample's
  * rank is the number of samples before it that the other gene has too.  So every gene is sorted once per
  * matrix (k_gene_order), and a pair costs two walks of S / 32 warp steps instead of two sorting networks:
- * 262,144 pairs of 1,000 samples (10 % missing) 32.8 -> 5 to 6 ms, three quarters of it the pairs of the next
- * paragraph.
+ * 262,144 pairs of 1,000 samples (10 % missing) 32.8 -> 1.7 ms, half of it the pairs of the next paragraph.
  *
  * Where two equal values of a gene both take part, their order comes from the network's swaps; the walk
- * finds such pairs (a flag per sample: equal to the next in order) and gives them to the network.
+ * finds such pairs (a flag per sample: equal to the next in order) and lists them for a launch of their own,
+ * a network per CTA of one warp in shared memory.  (In the walking warps they took 4 ms of 5: a gene with a
+ * repeated value gives a run of them to one warp.)
  */
 constexpr int ORDER_THREADS = 256;
 constexpr int ORDER_MOST = 8192;            /* samples k_gene_order sorts in shared memory (64 KB of keys) */
@@ -457,26 +458,11 @@ bool sim_spearman_orders_fit(const DevParams& P)
    return P.clus == 0 && P.corr >= 1 && P.S <= ORDER_MOST;
 }
 
-/* CTAs per SM that get room for the network's buffers */
-static int spearman_ctas(const DevParams& P)
+size_t sim_spearman_orders_bytes(const DevParams& P, char* base, SpearmanOrders* out)
 {
-   const int64_t cta = (int64_t)SPEARMAN_WARPS * 2 * P.P2 * (int)sizeof(float);
-   return (int)std::max<int64_t>(1, std::min<int64_t>(6, 2 * 1024 * 1024 / cta));
-}
-
-size_t sim_spearman_orders_bytes(int sms, const DevParams& P, char* base, SpearmanOrders* out)
-{
-   size_t off = 0;
-   auto take = [&](size_t bytes) {
-      char* p = base + off;
-      off += (bytes + 255) & ~(size_t)255;
-      return p;
-   };
-   uint16_t* order = (uint16_t*)take((size_t)P.G * P.S * sizeof(uint16_t));
-   uint8_t* ties = (uint8_t*)take((size_t)P.G);
-   float* buf = (float*)take((size_t)sms * spearman_ctas(P) * SPEARMAN_WARPS * 2 * P.P2 * sizeof(float));
-   if ( out ) *out = SpearmanOrders { order, ties, buf };
-   return off;
+   const size_t order = ((size_t)P.G * P.S * sizeof(uint16_t) + 255) & ~(size_t)255;
+   if ( out ) *out = SpearmanOrders { (uint16_t*)base, (uint8_t*)(base + order) };
+   return order + (size_t)P.G;
 }
 
 cudaError_t sim_spearman_orders(cudaStream_t st, const DevParams& P, const DevData& D, const SpearmanOrders& R)
@@ -546,7 +532,7 @@ __device__ __forceinline__ int spearman_walk(const uint16_t* __restrict__ order,
 }
 
 __global__ void __launch_bounds__(SPEARMAN_WARPS * 32)
-k_spearman_orders(DevParams P, DevData D, DevBlock B, SpearmanOrders R, int warp_bytes, int per_warp)
+k_spearman_orders(DevParams P, DevData D, DevBlock B, SpearmanOrders R, int32_t* tied_pairs, int warp_bytes, int per_warp)
 {
    extern __shared__ __align__(16) unsigned char spearman_smem[];
    const int lane = threadIdx.x & 31;
@@ -554,7 +540,6 @@ k_spearman_orders(DevParams P, DevData D, DevBlock B, SpearmanOrders R, int warp
    unsigned char* base = spearman_smem + (size_t)warp * warp_bytes;
    uint32_t* mask = (uint32_t*)base;                                     /* samples that both genes have */
    uint16_t* ranks = (uint16_t*)(base + ((P.W * 4 + 15) & ~15));         /* by x */
-   float* buf = R.buf + ((size_t)blockIdx.x * SPEARMAN_WARPS + warp) * 2 * P.P2;
    const int c = P.corr == 2 ? 1 : 0;
    const float nan = __int_as_float(0x7fc00000);
    const int64_t step = (int64_t)gridDim.x * SPEARMAN_WARPS * per_warp;
@@ -600,10 +585,8 @@ k_spearman_orders(DevParams P, DevData D, DevBlock B, SpearmanOrders R, int warp
                spearman_walk<true>(R.order + (size_t)y * P.S, P.S, mask, lane, tied, add);
             else
                spearman_walk<false>(R.order + (size_t)y * P.S, P.S, mask, lane, tied, add);
-            if ( tied )
-               r = spearman_network(D.gem + (size_t)x * P.S, D.gem + (size_t)y * P.S, P.S, mask, buf, lane);
-            else
-               r = spearman_value(__reduce_add_sync(0xffffffffu, diff), n);
+            r = spearman_value(__reduce_add_sync(0xffffffffu, diff), n);
+            if ( tied && lane == 0 ) tied_pairs[atomicAdd(B.tiles, 1ull)] = (int32_t)q;
          }
          __syncwarp();
          float* row = B.outCorr ? B.outCorr + q * P.max_k * P.ncorr : nullptr;
@@ -628,21 +611,46 @@ k_spearman_orders(DevParams P, DevData D, DevBlock B, SpearmanOrders R, int warp
    }
 }
 
-cudaError_t sim_launch_spearman(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B,
-                                const SpearmanOrders& R)
+/* the pairs whose ranks the network decides, one per warp (and CTA) */
+__global__ void __launch_bounds__(32) k_spearman_ties(DevParams P, DevData D, DevBlock B, const int32_t* tied_pairs)
 {
-   const int bytes = ((P.W * 4 + 15) & ~15) + ((P.S * 2 + 15) & ~15);
-   const int smem = bytes * SPEARMAN_WARPS;
+   extern __shared__ __align__(16) unsigned char spearman_smem[];
+   const int lane = threadIdx.x;
+   uint32_t* mask = (uint32_t*)spearman_smem;
+   float* buf = (float*)(spearman_smem + ((P.W * 4 + 15) & ~15));
+   const int64_t count = (int64_t)*B.tiles;
+   for ( int64_t i = blockIdx.x; i < count; i += gridDim.x )
+   {
+      const int64_t q = tied_pairs[i];
+      int32_t x, y;
+      pair_xy(B.start + q, x, y);
+      for ( int w = lane; w < P.W; w += 32 ) mask[w] = __ldg(D.umask + (size_t)x * P.W + w) & __ldg(D.umask + (size_t)y * P.W + w);
+      __syncwarp();
+      const float r = spearman_network(D.gem + (size_t)x * P.S, D.gem + (size_t)y * P.S, P.S, mask, buf, lane);
+      if ( lane == 0 && B.outCorr ) B.outCorr[q * P.max_k * P.ncorr + (P.corr == 2 ? 1 : 0)] = r;
+      __syncwarp();
+   }
+}
+
+cudaError_t sim_launch_spearman(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B,
+                                const SpearmanOrders& R, int32_t* tied_pairs)
+{
+   const int mask = (P.W * 4 + 15) & ~15;
+   const int bytes = mask + ((P.S * 2 + 15) & ~15);
+   const int smem = bytes * SPEARMAN_WARPS, net = mask + 2 * P.P2 * (int)sizeof(float);
+   int per_sm = 1, net_per_sm = 1;
    cudaError_t e = cudaFuncSetAttribute(k_spearman_orders, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-   int per_sm = 1;
+   if ( e == cudaSuccess ) e = cudaFuncSetAttribute(k_spearman_ties, cudaFuncAttributeMaxDynamicSharedMemorySize, net);
    if ( e == cudaSuccess )
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spearman_orders, SPEARMAN_WARPS * 32, smem);
+   if ( e == cudaSuccess ) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&net_per_sm, k_spearman_ties, 32, net);
    if ( e != cudaSuccess ) return e;
-   int64_t grid = (int64_t)sms * std::max(1, std::min(per_sm, spearman_ctas(P)));
+   int64_t grid = (int64_t)sms * std::max(1, per_sm);
    /* neighbouring pairs share x, so a warp takes up to 8 of them -- fewer if the warps would run out */
    const int per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(8, B.size / (grid * SPEARMAN_WARPS * 4)));
    grid = std::min(grid, (B.size + SPEARMAN_WARPS * per_warp - 1) / (SPEARMAN_WARPS * per_warp));
-   k_spearman_orders<<<(int)grid, SPEARMAN_WARPS * 32, smem, st>>>(P, D, B, R, bytes, per_warp);
+   k_spearman_orders<<<(int)grid, SPEARMAN_WARPS * 32, smem, st>>>(P, D, B, R, tied_pairs, bytes, per_warp);
+   k_spearman_ties<<<(int)std::min<int64_t>(B.size, (int64_t)sms * std::max(1, net_per_sm)), 32, net, st>>>(P, D, B, tied_pairs);
    return cudaGetLastError();
 }
 
