@@ -39,17 +39,35 @@ size_t sim_gmm_pairs_scratch(int sms, const DevParams& P, int n_cap, char* base,
    return labels + (size_t)sms * GP_WARPS * gp_global_floats(n_cap, P.max_k) * sizeof(float);
 }
 
-cudaError_t sim_launch_gmm_pairs(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevScratch& W,
-                                 const DevBlock& B, int n_cap)
+template <int WARPS>
+static cudaError_t launch(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevScratch& W,
+                          const DevBlock& B, int n_cap)
 {
    const int rows = gp_sort_rows(P);
    const int slot = gp_slot_floats(std::max(n_cap, 1), P.max_k, rows, false) * (int)sizeof(float);
-   const int smem = (int)std::min<int64_t>(GP_SMEM, (int64_t)slot * GP_WARPS);
-   const cudaError_t e = cudaFuncSetAttribute(k_gmm_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM);
+   const int smem = (int)std::min<int64_t>(GP_SMEM, (int64_t)slot * WARPS);
+   const cudaError_t e = cudaFuncSetAttribute(k_gmm_pairs<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM);
    if ( e != cudaSuccess ) return e;
    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(B.size, sms));
-   k_gmm_pairs<<<grid, GP_WARPS * 32, smem, st>>>(P, D, W, B, smem / (int)sizeof(float), rows, n_cap);
+   k_gmm_pairs<WARPS><<<grid, WARPS * 32, smem, st>>>(P, D, W, B, smem / (int)sizeof(float), rows, n_cap);
    return cudaGetLastError();
+}
+
+cudaError_t sim_launch_gmm_pairs(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevScratch& W,
+                                 const DevBlock& B, int n_cap)
+{
+   /*
+    * 16 warps of 128 registers (the K = 5 fit then reads its E step's parameters per chunk) or 12 of 168, by the
+    * pairs an SM holds with vg in shared memory and in global memory; thousands of pairs per second:
+    *   N = 122 (15 / 16): 1,030 / 981     N = 243 (12 / 16): 577 / 616
+    *   N = 423 (10 / 16): 350 / 303       N = 810 (6 / 11): 174 / 187
+    * and 12 where the block gives an SM no more.
+    */
+   const int rows = gp_sort_rows(P), n = std::max(n_cap, 1);
+   const int shared = GP_SMEM / (gp_slot_floats(n, P.max_k, rows, false) * (int)sizeof(float));
+   const int global = GP_SMEM / (gp_slot_floats(n, P.max_k, rows, true) * (int)sizeof(float));
+   const bool many = B.size > (int64_t)sms * GP_WARPS_FEW && (shared >= 14 || (shared < 11 && global >= 13));
+   return many ? launch<GP_WARPS>(sms, st, P, D, W, B, n_cap) : launch<GP_WARPS_FEW>(sms, st, P, D, W, B, n_cap);
 }
 
 } /* namespace kinc */

@@ -36,8 +36,13 @@
 
 namespace kinc {
 
-constexpr int GP_WARPS = 12;                /* warps (pairs) per SM at most: 168 registers each */
-constexpr int GP_SHARED_PAIRS = 9;          /* fewer pairs than this an SM: vg moves to global memory */
+constexpr int GP_WARPS = 16;                /* warps (pairs) per SM at most: 128 registers each */
+constexpr int GP_WARPS_FEW = 12;            /* at most, where no more pairs fit an SM: 168 registers each */
+/* fewer pairs than this an SM with vg in shared memory: it moves to global memory */
+__host__ __device__ constexpr int gp_shared_pairs(int warps)
+{
+   return warps == GP_WARPS_FEW ? 9 : 13;
+}
 constexpr int GP_CHUNK = 64;                /* samples the warp computes in one packed operation, and lays out
                                                as term rows together */
 constexpr int GP_ROW = GP_CHUNK + 4;        /* floats of a term row: rows start 4 banks apart, so the 16-byte
@@ -342,19 +347,29 @@ __device__ __forceinline__ F2 gp_density(F2 x0, F2 x1, F2 m0, F2 m1, F2 a, F2 b,
 
 /*
  * E step for finite parameters and samples: log p(x) of every sample, log(gamma/pi) (into vg), and
- * each component's largest log(gamma/pi) (into par).
+ * each component's largest log(gamma/pi) (into par).  KEEP: the parameters stay in registers, 14 for each
+ * component; else they are read again for every chunk.
  */
-template <int K, bool G>
+template <int K, bool G, bool KEEP>
 __device__ __forceinline__ void gp_e_step(const GpView& s, const GpLogTable& lt, int lane)
 {
    const F2 z = f2(s.nz);
    F2 q[K][7];
    float ga[K], gb[K];
+   auto parameters = [&](int k) {
+#pragma unroll
+      for ( int i = 0; i < 3; ++i )
+      {
+         const float4 v = *reinterpret_cast<const float4*>(s.par + k * GP_PAR + 4 * i);
+         q[k][2 * i] = f2(v.x, v.y);
+         q[k][2 * i + 1] = f2(v.z, v.w);
+      }
+      q[k][6] = gp_ld2(s.par + k * GP_PAR + 12);
+   };
 #pragma unroll
    for ( int k = 0; k < K; ++k )
    {
-#pragma unroll
-      for ( int i = 0; i < 7; ++i ) q[k][i] = gp_ld2(s.par + k * GP_PAR + 2 * i);
+      if ( KEEP ) parameters(k);
       ga[k] = -INFINITY;
       gb[k] = -INFINITY;
    }
@@ -373,6 +388,7 @@ __device__ __forceinline__ void gp_e_step(const GpView& s, const GpLogTable& lt,
 #pragma unroll
       for ( int k = 0; k < K; ++k )
       {
+         if ( !KEEP ) parameters(k);
          lg[k] = gp_density(x0, x1, q[k][0], q[k][1], q[k][2], q[k][3], q[k][4], q[k][5], z);
          lp[k] = q[k][6] + lg[k];
          float a, b;
@@ -487,8 +503,9 @@ struct GpM2Terms
  * The terms of chunk after chunk and, interleaved with them, the ordered sums of the chunk before:
  * beside each component's terms a K-th of the earlier chunk's 64 samples are added.  The sums are one
  * chain of dependent additions per row and the terms independent arithmetic, so each hides the
- * other's latency; two sets of rows alternate.  What a component reads is loaded one component ahead
- * (the stores of one may not be passed by the loads of the next); from global memory, one chunk ahead.  `lik`: this lane sums s.lpx
+ * other's latency; two sets of rows alternate.  The samples to add beside a component's terms are loaded before
+ * those, its vg one component ahead (the stores of one may not be passed by the loads of the next), or
+ * from global memory one chunk ahead.  `lik`: this lane sums s.lpx
  * instead of a term row.  Returns this lane's sum.
  */
 template <int K, bool G, class Terms>
@@ -509,9 +526,9 @@ __device__ __forceinline__ float gp_terms_and_sums(const GpView& s, bool lik, bo
    int flag[4];
 #pragma unroll
    for ( int i = 0; i < 4; ++i ) flag[i] = (act ? 1 : 0) + (zero >> i);
-   float4 v[2][GM];
+   float4 v[GM];
 #pragma unroll
-   for ( int g = 0; g < GM; ++g ) v[0][g] = v[1][g] = make_float4(0.f, 0.f, 0.f, 0.f);
+   for ( int g = 0; g < GM; ++g ) v[g] = make_float4(0.f, 0.f, 0.f, 0.f);
    float acc = 0.f;
    float* out = s.terms + 2 * lane;
    const float* in = s.x + 4 * lane;
@@ -539,25 +556,26 @@ __device__ __forceinline__ float gp_terms_and_sums(const GpView& s, bool lik, bo
          }
       }
       auto load = [&](int k) {
-         if ( !G ) val[k] = gp_ldv<G>(pv + k * s.n64);
 #pragma unroll
          for ( int g = NG * k / K; g < NG * (k + 1) / K; ++g )
-            gp_lds4(v[k & 1][g - NG * k / K], from + 16 * g, flag[g & 3]);
+            gp_lds4(v[g - NG * k / K], from + 16 * g, flag[g & 3]);
       };
+      if ( !G ) val[0] = gp_ldv<G>(pv);
       load(0);
 #pragma unroll
       for ( int k = 0; k < K; ++k )
       {
-         if ( k + 1 < K ) load(k + 1);
+         if ( !G && k + 1 < K ) val[k + 1] = gp_ldv<G>(pv + (k + 1) * s.n64);
          t[k].store(val[k], x0, x1, pv + k * s.n64, out + k * GP_ROW, K * GP_ROW);
 #pragma unroll
          for ( int g = 0; g < NG * (k + 1) / K - NG * k / K; ++g )
          {
-            acc += v[k & 1][g].x;
-            acc += v[k & 1][g].y;
-            acc += v[k & 1][g].z;
-            acc += v[k & 1][g].w;
+            acc += v[g].x;
+            acc += v[g].y;
+            acc += v[g].z;
+            acc += v[g].w;
          }
+         if ( k + 1 < K ) load(k + 1);
       }
       /* the first chunk's sums were of nothing; log p(x) starts over */
       acc = c == 0 ? 0.f : acc;
@@ -656,7 +674,7 @@ struct GpFit
  * E step is repeated then (its parameters are still in par) to give the label pass what the
  * reference's loggamma array holds.
  */
-template <int K, bool G>
+template <int K, bool G, int WARPS>
 __device__ __noinline__ GpFit gp_fit(GpLayout lay, double c2, bool ocl, bool icl, bool xsafe, int draws, int lane)
 {
    GpView s = lay.view();
@@ -711,7 +729,7 @@ __device__ __noinline__ GpFit gp_fit(GpLayout lay, double c2, bool ocl, bool icl
          __syncwarp();
       }
       if ( safe )
-         gp_e_step<K, G>(s, lt, lane);
+         gp_e_step<K, G, WARPS == GP_WARPS_FEW || K <= 3>(s, lt, lane);
       else
          gp_e_step_any(s, K, lane);
       if ( converged ) break;
@@ -836,7 +854,8 @@ __device__ __forceinline__ void gp_cta_sync(int warps)
  * full 100 iterations, so little is waited for).  When there are fewer pairs than slots, the groups
  * are smaller and every SM gets some.
  */
-__global__ void __launch_bounds__(GP_WARPS * 32, 1)
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
 k_gmm_pairs(DevParams P, DevData D, DevScratch W, DevBlock B, int smem_floats, int sort_rows, int n_cap)
 {
    extern __shared__ __align__(16) float gp_shared[];
@@ -844,10 +863,10 @@ k_gmm_pairs(DevParams P, DevData D, DevScratch W, DevBlock B, int smem_floats, i
    const int warp = threadIdx.x >> 5;
    const int n_most = B.order ? min(n_cap, B.N[B.start + B.order[0] - B.lo]) : n_cap;
    /* log(gamma/pi) in shared memory where that still leaves enough pairs to an SM */
-   const bool in_global = smem_floats / gp_slot_floats(max(n_most, 1), P.max_k, sort_rows, false) < GP_SHARED_PAIRS;
+   const bool in_global = smem_floats / gp_slot_floats(max(n_most, 1), P.max_k, sort_rows, false) < gp_shared_pairs(WARPS);
    const int slot_floats = gp_slot_floats(max(n_most, 1), P.max_k, sort_rows, in_global);
    const int64_t per_cta = (B.size + gridDim.x - 1) / gridDim.x;
-   const int slots = min(GP_WARPS, smem_floats / slot_floats);
+   const int slots = min(WARPS, smem_floats / slot_floats);
    const int warps = per_cta < slots ? (int)per_cta : slots;
    if ( warp >= warps ) return;
    const int64_t groups = (B.size + warps - 1) / warps;
@@ -925,11 +944,11 @@ k_gmm_pairs(DevParams P, DevData D, DevScratch W, DevBlock B, int smem_floats, i
             constexpr bool G = decltype(g)::value;
             switch ( k )
             {
-            case 1: return gp_fit<1, G>(l, P.c2, ocl, icl, xsafe, draw, lane);
-            case 2: return gp_fit<2, G>(l, P.c2, ocl, icl, xsafe, draw, lane);
-            case 3: return gp_fit<3, G>(l, P.c2, ocl, icl, xsafe, draw, lane);
-            case 4: return gp_fit<4, G>(l, P.c2, ocl, icl, xsafe, draw, lane);
-            default: return gp_fit<5, G>(l, P.c2, ocl, icl, xsafe, draw, lane);
+            case 1: return gp_fit<1, G, WARPS>(l, P.c2, ocl, icl, xsafe, draw, lane);
+            case 2: return gp_fit<2, G, WARPS>(l, P.c2, ocl, icl, xsafe, draw, lane);
+            case 3: return gp_fit<3, G, WARPS>(l, P.c2, ocl, icl, xsafe, draw, lane);
+            case 4: return gp_fit<4, G, WARPS>(l, P.c2, ocl, icl, xsafe, draw, lane);
+            default: return gp_fit<5, G, WARPS>(l, P.c2, ocl, icl, xsafe, draw, lane);
             }
          };
          f = in_global ? fit(std::true_type()) : fit(std::false_type());
