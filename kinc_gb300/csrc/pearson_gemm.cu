@@ -147,20 +147,26 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes)
    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
+/* whether phase `parity` of an mbarrier has completed (now or within the hardware's own short wait) */
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
+{
+   uint32_t ok;
+   asm volatile("{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok)
+                : "r"(bar), "r"(parity)
+                : "memory");
+   return ok != 0;
+}
+
 /* bounded wait for phase `parity` of an mbarrier; false on expiry */
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
 {
    const long long t0 = clock64();
    for ( ;; )
    {
-      uint32_t ok;
-      asm volatile("{\n\t.reg .pred p;\n\t"
-                   "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                   "selp.u32 %0, 1, 0, p;\n\t}"
-                   : "=r"(ok)
-                   : "r"(bar), "r"(parity)
-                   : "memory");
-      if ( ok ) return true;
+      if ( mbar_try(bar, parity) ) return true;
       if ( clock64() - t0 > WAIT_CYCLES ) return false;
    }
 }
@@ -365,6 +371,13 @@ __device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t* r)
                 : "r"(taddr));
 }
 
+__device__ __forceinline__ void tmem_ld8_async(uint32_t taddr, uint32_t* r)
+{
+   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                : "r"(taddr));
+}
+
 __device__ __forceinline__ void tmem_wait_ld()
 {
    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -500,33 +513,39 @@ __device__ __forceinline__ float diff_of_products(float a, float b, float c, flo
    return dop + err;
 }
 
-/* MMAs of one K-chunk in ring stage `stage` (see the TF32 / 3xBF16 notes above); acc0: 0 on the
- * tile's first chunk (the accumulators start from zero) */
-template <int MODE>
+/*
+ * MMAs of the K-steps K0 .. K1-1 of one K-chunk in ring stage `stage` (see the TF32 / 3xBF16 notes above);
+ * first: the tile's first chunk (the accumulators start from zero).  The queue of MMAs is short, so whatever the
+ * issuing thread does between two of them shows: every descriptor is the stage's own plus a constant (descriptors
+ * hold addresses in 16-byte units in their low bits, and a stage never crosses the field).
+ */
+template <int MODE, int K0 = 0, int K1 = Cfg<MODE>::BK / Cfg<MODE>::UMMA_K>
 __device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t stage, bool first)
 {
    using C = Cfg<MODE>;
    using L = Layout<MODE>;
    constexpr int BN = C::BN;
-   const uint32_t ysb = stage + C::NMAT * L::XMAT;
+   constexpr uint32_t Y = C::NMAT * L::XMAT;        /* the y-side operands begin here */
+   const uint64_t desc = smem_desc<MODE>(stage);
+   auto at = [&](uint32_t bytes) { return desc + (bytes >> 4); };
 #pragma unroll
-   for ( int ks = 0; ks < C::BK / C::UMMA_K; ++ks )
+   for ( int ks = K0; ks < K1; ++ks )
    {
       const uint32_t koff = ks * C::UMMA_K * C::ELEM;   /* byte step along K inside the row */
       const uint32_t acc = (!first || ks > 0) ? 1u : 0u;
       if ( merged<MODE>() && MODE == 2 )
       {
          /* x side: 0 Ah, 1 Al, 2 Qh, 3 Ql, 4 M; y side in slots [Ql][Qh][Ah][M][Al] */
-         const uint64_t xah = smem_desc<MODE>(stage + 0 * L::XMAT + koff);
-         const uint64_t xal = smem_desc<MODE>(stage + 1 * L::XMAT + koff);
-         const uint64_t xqh = smem_desc<MODE>(stage + 2 * L::XMAT + koff);
-         const uint64_t xql = smem_desc<MODE>(stage + 3 * L::XMAT + koff);
-         const uint64_t xm = smem_desc<MODE>(stage + 4 * L::XMAT + koff);
-         const uint64_t y_ql = smem_desc<MODE>(ysb + 0 * L::YMAT + koff);
-         const uint64_t y_qh_ah_m = smem_desc<MODE>(ysb + 1 * L::YMAT + koff);
-         const uint64_t y_ah_m_al = smem_desc<MODE>(ysb + 2 * L::YMAT + koff);
-         const uint64_t y_m = smem_desc<MODE>(ysb + 3 * L::YMAT + koff);
-         const uint64_t y_al = smem_desc<MODE>(ysb + 4 * L::YMAT + koff);
+         const uint64_t xah = at(0 * L::XMAT + koff);
+         const uint64_t xal = at(1 * L::XMAT + koff);
+         const uint64_t xqh = at(2 * L::XMAT + koff);
+         const uint64_t xql = at(3 * L::XMAT + koff);
+         const uint64_t xm = at(4 * L::XMAT + koff);
+         const uint64_t y_ql = at(Y + 0 * L::YMAT + koff);
+         const uint64_t y_qh_ah_m = at(Y + 1 * L::YMAT + koff);
+         const uint64_t y_ah_m_al = at(Y + 2 * L::YMAT + koff);
+         const uint64_t y_m = at(Y + 3 * L::YMAT + koff);
+         const uint64_t y_al = at(Y + 4 * L::YMAT + koff);
          mma<MODE, 3 * BN>(tmem + 0, xah, y_ah_m_al, acc);      /* Sxy(hh) | Sx(h) | Sxy(hl) */
          mma<MODE, 2 * BN>(tmem + 0, xal, y_ah_m_al, 1u);       /* += Sxy(lh) | Sx(l) */
          mma<MODE, BN>(tmem + acc_col<MODE>(3), xqh, y_m, acc); /* Sxx */
@@ -537,12 +556,12 @@ __device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t stage, bool 
       }
       else if ( merged<MODE>() )
       {
-         const uint64_t xa = smem_desc<MODE>(stage + 0 * L::XMAT + koff);
-         const uint64_t xq = smem_desc<MODE>(stage + 1 * L::XMAT + koff);
-         const uint64_t xm = smem_desc<MODE>(stage + 2 * L::XMAT + koff);
-         const uint64_t y_q_a_m = smem_desc<MODE>(ysb + 0 * L::YMAT + koff);   /* [A2_y; A_y; M_y] */
-         const uint64_t y_a_m = smem_desc<MODE>(ysb + 1 * L::YMAT + koff);     /* [A_y; M_y] */
-         const uint64_t y_m = smem_desc<MODE>(ysb + 2 * L::YMAT + koff);       /* M_y */
+         const uint64_t xa = at(0 * L::XMAT + koff);
+         const uint64_t xq = at(1 * L::XMAT + koff);
+         const uint64_t xm = at(2 * L::XMAT + koff);
+         const uint64_t y_q_a_m = at(Y + 0 * L::YMAT + koff);   /* [A2_y; A_y; M_y] */
+         const uint64_t y_a_m = at(Y + 1 * L::YMAT + koff);     /* [A_y; M_y] */
+         const uint64_t y_m = at(Y + 2 * L::YMAT + koff);       /* M_y */
          mma<MODE, 2 * BN>(tmem + acc_col<MODE>(0), xa, y_a_m, acc);     /* Sxy | Sx */
          mma<MODE, BN>(tmem + acc_col<MODE>(3), xq, y_m, acc);           /* Sxx */
          mma<MODE, 3 * BN>(tmem + acc_col<MODE>(4), xm, y_q_a_m, acc);   /* Syy | Sy | n */
@@ -550,12 +569,12 @@ __device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t stage, bool 
       else if ( MODE != 2 )
       {
          /* x side: 0 A, 1 A2, 2 M; y side likewise */
-         const uint64_t xa = smem_desc<MODE>(stage + 0 * L::XMAT + koff);
-         const uint64_t xq = smem_desc<MODE>(stage + 1 * L::XMAT + koff);
-         const uint64_t xm = smem_desc<MODE>(stage + 2 * L::XMAT + koff);
-         const uint64_t ya = smem_desc<MODE>(ysb + 0 * L::YMAT + koff);
-         const uint64_t yq = smem_desc<MODE>(ysb + 1 * L::YMAT + koff);
-         const uint64_t ym = smem_desc<MODE>(ysb + 2 * L::YMAT + koff);
+         const uint64_t xa = at(0 * L::XMAT + koff);
+         const uint64_t xq = at(1 * L::XMAT + koff);
+         const uint64_t xm = at(2 * L::XMAT + koff);
+         const uint64_t ya = at(Y + 0 * L::YMAT + koff);
+         const uint64_t yq = at(Y + 1 * L::YMAT + koff);
+         const uint64_t ym = at(Y + 2 * L::YMAT + koff);
          mma<MODE>(tmem + 0 * BN, xa, ya, acc);   /* Sxy */
          mma<MODE>(tmem + 1 * BN, xa, ym, acc);   /* Sx */
          mma<MODE>(tmem + 2 * BN, xm, ya, acc);   /* Sy */
@@ -570,8 +589,8 @@ __device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t stage, bool 
 #pragma unroll
          for ( int m = 0; m < 5; ++m )
          {
-            xd[m] = smem_desc<MODE>(stage + m * L::XMAT + koff);
-            yd[m] = smem_desc<MODE>(ysb + m * L::YMAT + koff);
+            xd[m] = at(m * L::XMAT + koff);
+            yd[m] = at(Y + m * L::YMAT + koff);
          }
          mma<MODE>(tmem + 0 * BN, xd[0], yd[0], acc);   /* Sxy: hi.hi + hi.lo + lo.hi */
          mma<MODE>(tmem + 0 * BN, xd[0], yd[1], 1u);
@@ -692,8 +711,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
    {
       if ( lane == 0 )
       {
-         /* ---- MMA issuer */
-         int used = 0, tl = 0;
+         /* ---- MMA issuer.  It asks for the next chunk half-way through the MMAs of this one and looks at the
+          * answer after the rest: a wait between two chunks left the tensor core idle for about 150 clk of the
+          * chunk's 820 (the K-step of 16 samples with operands in place: 204 clk without waits, 243 with one per
+          * chunk, 218 asked for early). */
+         constexpr int KS = C::BK / C::UMMA_K;
+         int s = 0, tl = 0;
+         uint32_t phase = 0;
          for ( int t = blockIdx.x; t < ntiles && !*(volatile int*)&s_fail; t += gridDim.x, ++tl )
          {
             if ( tl > 0 && !mbar_wait(tempty, (tl - 1) & 1) )
@@ -702,18 +726,24 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            bool ok = true;
-            for ( int kc = 0; kc < K; ++kc, ++used )
+            bool ok = true, ready = false;
+            for ( int kc = 0; kc < K; ++kc )
             {
-               const int s = used % STAGES;
-               if ( !mbar_wait(full0 + 8 * s, (used / STAGES) & 1) )
+               if ( !ready && !mbar_wait(full0 + 8 * s, phase) )
                {
                   ok = false;
                   break;
                }
                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-               issue_chunk<MODE>(tmem, smem_u32(ring + s * L::STAGE), kc == 0);
+               const int next = s + 1 == STAGES ? 0 : s + 1;
+               const uint32_t next_phase = next == 0 ? phase ^ 1 : phase;
+               const uint32_t stage = smem_u32(ring + s * L::STAGE);
+               issue_chunk<MODE, 0, KS / 2>(tmem, stage, kc == 0);
+               ready = kc + 1 < K && mbar_try(full0 + 8 * next, next_phase);
+               issue_chunk<MODE, KS / 2, KS>(tmem, stage, kc == 0);
                mma_commit(empty0 + 8 * s);      /* frees the stage when these MMAs have read it */
+               s = next;
+               phase = next_phase;
             }
             if ( !ok )
             {
@@ -732,9 +762,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
        * next tile's MMAs instead of holding them up. */
       const int quarter = warp & 3;
       const int half = (warp - 2) >> 2;
-      constexpr int WCH = BN / 32;                 /* 16-column chunks per warp */
-      static_assert(BN % 32 == 0, "two warps share a quarter's columns");
-      const int c0 = half * WCH;
       float* ebuf = (float*)(ring + L::RING + 256) + (warp - 2) * (32 * 8);
       int tl = 0;
       for ( int t = blockIdx.x; t < ntiles; t += gridDim.x, ++tl )
@@ -752,60 +779,68 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
          const int2 ij = tiles[t];
          const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
-         /* r of this lane's row (TMEM lane = pair row) and the warp's columns */
-         float r[WCH][16];
-         {
+         /* r of this lane's row (TMEM lane = pair row) and the warp's columns.  The next tile's MMAs wait for
+          * TMEM, so only a part of the columns is finished while the rest is still there: what fits beside the
+          * others' sums in registers (six or seven sums a column). */
+         constexpr int COLS = BN / 2, SUMS = sxy2_col<MODE>() >= 0 ? NACC + 1 : NACC;
+         constexpr int EARLY = SUMS > NACC ? 16 : 8;
+         float r[COLS];
+         auto load = [&](int c, int n8, uint32_t (*v)[COLS]) {
 #pragma unroll
-            for ( int w = 0; w < WCH; ++w )
+            for ( int i = 0; i < n8; ++i )
             {
-               const int c = c0 + w;
-               /* all of the chunk's accumulators in flight at once, then one wait */
-               uint32_t v[NACC + 1][16];
 #pragma unroll
-               for ( int a = 0; a < NACC; ++a ) tmem_ld16_async(lane_base + acc_col<MODE>(a) + c * 16, v[a]);
+               for ( int a = 0; a < NACC; ++a )
+                  tmem_ld8_async(lane_base + acc_col<MODE>(a) + half * COLS + c + 8 * i, &v[a][c + 8 * i]);
                if constexpr ( sxy2_col<MODE>() >= 0 )
-                  tmem_ld16_async(lane_base + (uint32_t)sxy2_col<MODE>() + c * 16, v[NACC]);
-               tmem_wait_ld();
-#pragma unroll
-               for ( int jj = 0; jj < 16; ++jj )
-               {
-                  float sxy = __uint_as_float(v[0][jj]);
-                  if constexpr ( sxy2_col<MODE>() >= 0 ) sxy += __uint_as_float(v[NACC][jj]);
-                  const float sx = __uint_as_float(v[1][jj]), sy = __uint_as_float(v[2][jj]);
-                  const float sxx = __uint_as_float(v[3][jj]), syy = __uint_as_float(v[4][jj]);
-                  const float n = __uint_as_float(v[5][jj]);
-                  r[w][jj] = __int_as_float(0x7fc00000);
-                  if ( n >= (float)args.min_samples && n > 0.f )
-                  {
-                     const float num = diff_of_products(n, sxy, sx, sy);
-                     const float dx = diff_of_products(n, sxx, sx, sx);
-                     const float dy = diff_of_products(n, syy, sy, sy);
-                     r[w][jj] = num * rsqrtf(dx) * rsqrtf(dy);
-                  }
-               }
+                  tmem_ld8_async(lane_base + (uint32_t)sxy2_col<MODE>() + half * COLS + c + 8 * i, &v[NACC][c + 8 * i]);
             }
-         }
-         /* every TMEM read of this warp is complete (tmem_wait_ld): hand TMEM back */
+         };
+         auto finish = [&](int j, uint32_t (*v)[COLS]) {
+            float sxy = __uint_as_float(v[0][j]);
+            if constexpr ( sxy2_col<MODE>() >= 0 ) sxy += __uint_as_float(v[NACC][j]);
+            const float sx = __uint_as_float(v[1][j]), sy = __uint_as_float(v[2][j]);
+            const float sxx = __uint_as_float(v[3][j]), syy = __uint_as_float(v[4][j]);
+            const float n = __uint_as_float(v[5][j]);
+            r[j] = __int_as_float(0x7fc00000);
+            if ( n >= (float)args.min_samples && n > 0.f )
+            {
+               const float num = diff_of_products(n, sxy, sx, sy);
+               const float dx = diff_of_products(n, sxx, sx, sx);
+               const float dy = diff_of_products(n, syy, sy, sy);
+               r[j] = num * rsqrtf(dx) * rsqrtf(dy);
+            }
+         };
+         uint32_t v[SUMS][COLS];
+         load(0, EARLY / 8, v);
+         tmem_wait_ld();
+#pragma unroll
+         for ( int j = 0; j < EARLY; ++j ) finish(j, v);
+         load(EARLY, (COLS - EARLY) / 8, v);
+         tmem_wait_ld();
+         /* every TMEM read of this warp is complete: hand TMEM back */
          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
          __syncwarp();
          if ( lane == 0 ) mbar_arrive(tempty);
+#pragma unroll
+         for ( int j = EARLY; j < COLS; ++j ) finish(j, v);
          /* written through a 32 x 8 shared-memory tile so that each store covers 8 neighbouring
           * pairs of 4 rows (a lane's own row would put the warp's 32 stores in 32 rows); element
           * (row, col) sits at row * 8 + (col ^ (row / 4)), conflict-free both ways */
          const int64_t x0 = (int64_t)ij.x * BM + quarter * 32;   /* the warp's first row */
 #pragma unroll
-         for ( int g = 0; g < 2 * WCH; ++g )
+         for ( int g = 0; g < COLS / 8; ++g )
          {
             __syncwarp();
 #pragma unroll
-            for ( int j = 0; j < 8; ++j ) ebuf[lane * 8 + (j ^ (lane >> 2))] = r[g >> 1][(g & 1) * 8 + j];
+            for ( int j = 0; j < 8; ++j ) ebuf[lane * 8 + (j ^ (lane >> 2))] = r[g * 8 + j];
             __syncwarp();
 #pragma unroll
             for ( int i = 0; i < 8; ++i )
             {
                const int rr = 4 * i + (lane >> 3), cc = lane & 7;
                const int64_t x = x0 + rr;
-               const int64_t y = (int64_t)ij.y * BN + c0 * 16 + g * 8 + cc;
+               const int64_t y = (int64_t)ij.y * BN + half * COLS + g * 8 + cc;
                const int64_t p = x * (x - 1) / 2 + y;
                if ( x < args.G && y < x && p >= args.start && p < args.end )
                   args.out_corr[(p - args.start) * args.max_k] = ebuf[rr * 8 + (cc ^ i)];
