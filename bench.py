@@ -548,7 +548,7 @@ def rmt_leg(blocks=1000, size=5, cpu=True):
     """RMT thresholding (include/kinc_rmt.h) with the reference's defaults except a 0.01 threshold step,
     on a clique network of blocks x size genes (kinc_gb300.synthetic.clique_network): pruned matrices
     grow to a few thousand rows before the spacing test finds the threshold.  GPU wall clock of the
-    whole analytic (pruned matrices in HBM, cuSOLVER eigenvalues, host unfolding) beside the oracle
+    whole analytic (pruned matrices in HBM, eigenvalues by connected components, host unfolding) beside the oracle
     (numpy eigensolver, scipy spline) on the host cores, with the step sequences compared."""
     from kinc_gb300 import synthetic
     from kinc_gb300.rmt import RMT
@@ -749,7 +749,7 @@ def main():
     achieved = units * FLOPS_PER_UNIT / (ms / 1e3) / 1e12
     traffic = None
     issue = None
-    tpath = os.path.join(REPO, "profiles", "k_similarity_traffic.json")
+    tpath = os.path.join(REPO, "profiles", "k_gmm_pairs_traffic.json")
     if os.path.exists(tpath):
         with open(tpath) as fh:
             tj = json.load(fh)
@@ -766,7 +766,7 @@ def main():
                 "frac": achieved / fp32_peak, "traffic": traffic,
                 "peak_source": f"nominal FP32 FMA rate: {props.multi_processor_count} SMs x 128 lanes x 2 flops x "
                                f"{sm_max:.0f} MHz (MEASURED_PEAKS.json holds no FP32 figure)",
-                "kernel": "k_similarity", "units": units, "flops_per_unit": FLOPS_PER_UNIT, "fits": fits,
+                "kernel": "k_gmm_pairs", "units": units, "flops_per_unit": FLOPS_PER_UNIT, "fits": fits,
                 "issue_frac": issue["frac"] if issue else None, "issue": issue}
 
     tensor_core = None if args.no_dense else dense_leg(L, vp, args.dense_check_pairs)

@@ -19,7 +19,7 @@
  * outliers, Spearman), tile kernel -> this one: 1,128 pairs of 96 samples
  * 71.8 -> 1.9 ms, 32,768 pairs of 1,000 samples (N = 810) 580 -> 173 ms,
  * 131,072 pairs 1,131 -> 682 ms, 196,608 pairs of 500 samples (ICL, both
- * correlations) 947 -> 645 ms.
+ * correlations) 947 -> 561 ms.
  *
  * What bounds it: per 64 samples, component and iteration the fit needs 122
  * cycles of a scheduler's FP32 pipe (a packed FP32 instruction takes two; the
