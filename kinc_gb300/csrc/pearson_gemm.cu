@@ -514,22 +514,23 @@ __device__ __forceinline__ float diff_of_products(float a, float b, float c, flo
 }
 
 /*
- * MMAs of the K-steps K0 .. K1-1 of one K-chunk in ring stage `stage` (see the TF32 / 3xBF16 notes above);
- * first: the tile's first chunk (the accumulators start from zero).  The queue of MMAs is short, so whatever the
+ * MMAs of one K-chunk in ring stage `stage` (see the TF32 / 3xBF16 notes above); first: the tile's first chunk
+ * (the accumulators start from zero); ask() is called in front of the chunk's last wide MMA.  The queue of MMAs is short, so whatever the
  * issuing thread does between two of them shows: every descriptor is the stage's own plus a constant (descriptors
  * hold addresses in 16-byte units in their low bits, and a stage never crosses the field).
  */
-template <int MODE, int K0 = 0, int K1 = Cfg<MODE>::BK / Cfg<MODE>::UMMA_K>
-__device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t stage, bool first)
+template <int MODE, class F>
+__device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t stage, bool first, F&& ask)
 {
    using C = Cfg<MODE>;
    using L = Layout<MODE>;
    constexpr int BN = C::BN;
+   constexpr int KS = C::BK / C::UMMA_K;
    constexpr uint32_t Y = C::NMAT * L::XMAT;        /* the y-side operands begin here */
    const uint64_t desc = smem_desc<MODE>(stage);
    auto at = [&](uint32_t bytes) { return desc + (bytes >> 4); };
 #pragma unroll
-   for ( int ks = K0; ks < K1; ++ks )
+   for ( int ks = 0; ks < KS; ++ks )
    {
       const uint32_t koff = ks * C::UMMA_K * C::ELEM;   /* byte step along K inside the row */
       const uint32_t acc = (!first || ks > 0) ? 1u : 0u;
@@ -550,6 +551,7 @@ __device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t stage, bool 
          mma<MODE, 2 * BN>(tmem + 0, xal, y_ah_m_al, 1u);       /* += Sxy(lh) | Sx(l) */
          mma<MODE, BN>(tmem + acc_col<MODE>(3), xqh, y_m, acc); /* Sxx */
          mma<MODE, BN>(tmem + acc_col<MODE>(3), xql, y_m, 1u);
+         if ( ks == KS - 1 ) ask();
          mma<MODE, 3 * BN>(tmem + acc_col<MODE>(4), xm, y_qh_ah_m, acc);   /* Syy(h) | Sy(h) | n */
          mma<MODE, BN>(tmem + acc_col<MODE>(4), xm, y_ql, 1u);             /* Syy += l */
          mma<MODE, BN>(tmem + acc_col<MODE>(2), xm, y_al, 1u);             /* Sy += l */
@@ -564,6 +566,7 @@ __device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t stage, bool 
          const uint64_t y_m = at(Y + 2 * L::YMAT + koff);       /* M_y */
          mma<MODE, 2 * BN>(tmem + acc_col<MODE>(0), xa, y_a_m, acc);     /* Sxy | Sx */
          mma<MODE, BN>(tmem + acc_col<MODE>(3), xq, y_m, acc);           /* Sxx */
+         if ( ks == KS - 1 ) ask();
          mma<MODE, 3 * BN>(tmem + acc_col<MODE>(4), xm, y_q_a_m, acc);   /* Syy | Sy | n */
       }
       else if ( MODE != 2 )
@@ -711,11 +714,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
    {
       if ( lane == 0 )
       {
-         /* ---- MMA issuer.  It asks for the next chunk half-way through the MMAs of this one and looks at the
-          * answer after the rest: a wait between two chunks left the tensor core idle for about 150 clk of the
-          * chunk's 820 (the K-step of 16 samples with operands in place: 204 clk without waits, 243 with one per
-          * chunk, 218 asked for early). */
-         constexpr int KS = C::BK / C::UMMA_K;
+         /* ---- MMA issuer.  It asks for the next chunk in front of this chunk's last wide MMA (N = 192, 96 clk) and
+          * looks at the answer after it: a wait between two chunks left the tensor core idle for about 150 clk of
+          * the chunk's 820 (a K-step of 16 samples with operands in place: 204 clk without waits, 243 with one per
+          * chunk).  18M pairs of 2,000 samples, FP16: asked half-way through the chunk 311 us, before its last
+          * K-step 308, before its last wide MMA 303. */
          int s = 0, tl = 0;
          uint32_t phase = 0;
          for ( int t = blockIdx.x; t < ntiles && !*(volatile int*)&s_fail; t += gridDim.x, ++tl )
@@ -737,10 +740,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                const int next = s + 1 == STAGES ? 0 : s + 1;
                const uint32_t next_phase = next == 0 ? phase ^ 1 : phase;
-               const uint32_t stage = smem_u32(ring + s * L::STAGE);
-               issue_chunk<MODE, 0, KS / 2>(tmem, stage, kc == 0);
-               ready = kc + 1 < K && mbar_try(full0 + 8 * next, next_phase);
-               issue_chunk<MODE, KS / 2, KS>(tmem, stage, kc == 0);
+               ready = false;
+               issue_chunk<MODE>(tmem, smem_u32(ring + s * L::STAGE), kc == 0,
+                                 [&] { ready = kc + 1 < K && mbar_try(full0 + 8 * next, next_phase); });
                mma_commit(empty0 + 8 * s);      /* frees the stage when these MMAs have read it */
                s = next;
                phase = next_phase;
