@@ -75,7 +75,8 @@ int kinc_rmt_run(const char* cmx_path, int32_t little_endian, const kinc_rmt_par
 int kinc_rmt_chi_square(const float* eigens, int32_t n, const kinc_rmt_params* p, float* out_chi);
 
 /* Eigenvalues of the pruned matrix at one threshold, sorted by ascending |lambda|;
- * *size receives the pruned dimension (eigens must hold genes * max_clusters floats). */
+ * *size receives the pruned dimension (eigens must hold genes * max_clusters floats).  With an infinite
+ * correlation among the kept items all of them are NaN; NaN correlations are never kept. */
 int kinc_rmt_prune_eigenvalues(int32_t genes, int32_t max_clusters, int64_t n, const int32_t* x, const int32_t* y,
                                const int8_t* c, const float* r, float threshold, float* eigens, int32_t* size);
 

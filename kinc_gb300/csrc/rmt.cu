@@ -287,6 +287,7 @@ struct RmtDevice
 {
    int32_t G = 0, K = 0;
    int64_t n = 0;
+   bool infinite = false;              /* an item is infinite */
    int32_t *dx = nullptr, *dy = nullptr, *droot = nullptr, *dlist = nullptr, *dinfo = nullptr;
    int2* dplace = nullptr;
    RmtComponent* dcomp = nullptr;
@@ -327,6 +328,7 @@ int device_setup(RmtDevice& d, int32_t G, int32_t K, int64_t n, const int32_t* x
       if ( x[i] <= y[i] || y[i] < 0 || x[i] >= G || c[i] < 0 || c[i] >= K )
          return rmt_fail(KINC_SIM_EINVAL, "item %lld (%d, %d, %d) outside %d genes x %d clusters", (long long)i, x[i],
                          y[i], c[i], G, K);
+   d.infinite = std::any_of(r, r + n, [](float v) { return std::isinf(v); });
    d.G = G;
    d.K = K;
    d.n = n;
@@ -429,6 +431,14 @@ int device_eigenvalues(RmtDevice& d, float t, std::vector<float>& eig, int32_t& 
       d.place[(size_t)i] = p;
    }
    if ( m == 0 ) return KINC_SIM_OK;
+   if ( d.infinite )
+   {
+      /* every threshold keeps an infinite item, and a matrix with one has no eigenvalues.  The reference's dense
+       * solver turns all that it meets afterwards into NaN; here none are computed: bisection would return finite
+       * values (fmin and fmax drop the NaN that the reduction makes of an infinity) */
+      eig.assign((size_t)m, std::numeric_limits<float>::quiet_NaN());
+      return KINC_SIM_OK;
+   }
    size_t need = 0;
    int32_t values = 0, most[2] = { 0, 0 };
    for ( size_t k = 0; k < comp.size(); ++k )
@@ -479,9 +489,12 @@ int device_eigenvalues(RmtDevice& d, float t, std::vector<float>& eig, int32_t& 
    std::vector<double> w((size_t)m);
    RCK(cudaMemcpyAsync(w.data(), d.dW, (size_t)m * sizeof(double), cudaMemcpyDeviceToHost, d.st));
    RCK(cudaStreamSynchronize(d.st));
-   /* GSL_EIGEN_SORT_ABS_ASC: ascending |lambda| (ascending among equal magnitudes) */
-   std::sort(w.begin(), w.end());
-   std::stable_sort(w.begin(), w.end(), [](double a, double b) { return std::fabs(a) < std::fabs(b); });
+   /* GSL_EIGEN_SORT_ABS_ASC: ascending |lambda| (ascending among equal magnitudes); a NaN would come last */
+   std::sort(w.begin(), w.end(), [](double a, double b) {
+      if ( std::isnan(a) || std::isnan(b) ) return !std::isnan(a) && std::isnan(b);
+      const double fa = std::fabs(a), fb = std::fabs(b);
+      return fa != fb ? fa < fb : a < b;
+   });
    eig.resize((size_t)m);
    for ( int32_t i = 0; i < m; ++i ) eig[(size_t)i] = (float)w[(size_t)i];
    return KINC_SIM_OK;

@@ -77,3 +77,22 @@ def test_repeated_eigenvalues():
     same = (x // 10) == (y // 10)
     x, y = x[same].astype(np.int32), y[same].astype(np.int32)
     _check(50, 1, x, y, np.zeros(len(x), np.int8), np.full(len(x), 0.8, np.float32), 0.5)
+
+
+@pytest.mark.parametrize("rows,a,b,value", [(6, 5, 4, np.inf), (6, 1, 0, np.inf), (40, 39, 38, -np.inf), (150, 7, 3, np.inf)])
+def test_infinite_items_have_no_eigenvalues(rows, a, b, value):
+    """A matrix with an infinite element has no eigenvalues: every one is NaN, whichever component it is in, and a
+    search over thresholds, all of which keep such an item, finds none."""
+    G, x, y, c, r = _network([rows, 4, 9], "clique")
+    x, y = np.concatenate([x, [G + a]]).astype(np.int32), np.concatenate([y, [G + b]]).astype(np.int32)
+    more, less = np.tril_indices(rows, -1)                 # a clique of its own behind the others, with the item in it
+    other = (more != a) | (less != b)
+    x, y = np.concatenate([x, G + more[other]]).astype(np.int32), np.concatenate([y, G + less[other]]).astype(np.int32)
+    r = np.concatenate([r, [value], np.linspace(0.7, 0.9, other.sum())]).astype(np.float32)
+    c = np.zeros(len(x), np.int8)
+    keep = np.abs(r) >= np.float32(0.6)
+    got = RMT().prune_eigenvalues((x, y, c, r), G + rows, 1, 0.6)
+    assert len(got) == len(np.unique(np.concatenate([x[keep], y[keep]]))) and np.all(np.isnan(got))
+    threshold, steps = RMT(tstart=0.7, tstep=0.05, tstop=0.5).run(items=(x, y, c, r), genes=G + rows, max_clusters=1,
+                                                                  strict=False)
+    assert threshold is None and len(steps) >= 4 and np.all(steps[:, 2] == -1.0)
