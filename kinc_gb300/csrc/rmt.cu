@@ -82,7 +82,9 @@ __global__ void k_rmt_roots(int64_t rows, const unsigned int* __restrict__ mx, f
       root[i] = __uint_as_float(mx[i]) >= t ? (int32_t)i : -1;
 }
 
-/* the root of i, halving the path on the way (a root's parent is itself, any other's is smaller) */
+/* The root of i, halving the path on the way (a root's parent is itself, any other's is smaller).  Union-find with
+ * path halving and roots hung by compare-and-swap: R. J. Anderson, H. Woll, Wait-free parallel algorithms for the
+ * union-find problem, STOC 1991. */
 __device__ __forceinline__ int32_t rmt_find(volatile int32_t* root, int32_t i)
 {
    int32_t p = root[i];
@@ -121,10 +123,18 @@ __global__ void k_rmt_unite(int64_t n, int K, const int32_t* __restrict__ x, con
    }
 }
 
+/* every kept row's root.  No halving here: each entry has one writer, so what is left in it is the root (a
+ * neighbour's halving could put an older ancestor back). */
 __global__ void k_rmt_flatten(int64_t rows, int32_t* root)
 {
+   volatile const int32_t* parent = root;
    for ( int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x )
-      if ( root[i] >= 0 ) root[i] = rmt_find(root, (int32_t)i);
+   {
+      int32_t p = parent[i];
+      if ( p < 0 ) continue;
+      for ( int32_t g = parent[p]; g != p; g = parent[p] ) p = g;
+      root[i] = p;
+   }
 }
 
 /* a component: its rows, and where its matrix (row-major, lower triangle) and eigenvalues lie */
