@@ -69,7 +69,7 @@ __global__ void k_rmt_max(int64_t n, int K, const int32_t* __restrict__ x, const
  * Components.  The pruned matrix joins two rows only where an item is kept, and at the thresholds of a search most
  * rows sit in small groups; after a permutation the matrix is block diagonal, and its eigenvalues are the blocks'.
  * So the rows are united along the kept items, components of up to RMT_BLOCK rows are solved by k_rmt_blocks, all in
- * one launch, and only larger ones go to cuSOLVER, each by itself.  A 1,000-row matrix of 10-row components:
+ * one launch, and only larger ones go to cuSOLVER (rmt_plan: also where the whole matrix in one solve is faster).  A 1,000-row matrix of 10-row components:
  * 23.5 -> 0.7 ms; a search over 50 thresholds of 5,000 rows in 5-row components 10.5 -> 0.1 s.
  */
 constexpr int RMT_BLOCK = 128;              /* rows of a block k_rmt_blocks holds in shared memory (128 KB) */
@@ -137,14 +137,15 @@ __global__ void k_rmt_flatten(int64_t rows, int32_t* root)
    }
 }
 
-/* a component: its rows, and where its matrix (row-major, lower triangle) and eigenvalues lie */
+/* a matrix to solve (one component or several): its rows, and where it (row-major, lower triangle) and its eigenvalues
+ * lie */
 struct RmtComponent
 {
    int64_t at;
    int32_t size, values;
 };
 
-/* the unit diagonals and the kept items; place[row] = { component, position in it } */
+/* the unit diagonals and the kept items; place[row] = { matrix, position in it } */
 __global__ void k_rmt_fill(int64_t rows, int64_t n, int K, const int32_t* __restrict__ x, const int32_t* __restrict__ y,
                            const int8_t* __restrict__ c, const float* __restrict__ r, float t,
                            const int2* __restrict__ place, const RmtComponent* __restrict__ comp, double* __restrict__ A)
@@ -297,6 +298,7 @@ struct RmtDevice
 {
    int32_t G = 0, K = 0;
    int64_t n = 0;
+   int sms = 1;
    bool infinite = false;              /* an item is infinite */
    int32_t *dx = nullptr, *dy = nullptr, *droot = nullptr, *dlist = nullptr, *dinfo = nullptr;
    int2* dplace = nullptr;
@@ -343,6 +345,9 @@ int device_setup(RmtDevice& d, int32_t G, int32_t K, int64_t n, const int32_t* x
    d.K = K;
    d.n = n;
    const int64_t rows = (int64_t)G * K;
+   int dev = 0;
+   RCK(cudaGetDevice(&dev));
+   RCK(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
    RCK(cudaStreamCreateWithFlags(&d.st, cudaStreamNonBlocking));
    RCK(cudaMalloc(&d.dx, std::max<int64_t>(n, 1) * 4));
    RCK(cudaMalloc(&d.dy, std::max<int64_t>(n, 1) * 4));
@@ -372,8 +377,81 @@ int device_setup(RmtDevice& d, int32_t G, int32_t K, int64_t n, const int32_t* x
    return KINC_SIM_OK;
 }
 
-/* the eigenvalues of one component too large for k_rmt_blocks: from its matrix at dA + at into dW + values */
-int large_component(RmtDevice& d, const RmtComponent& q)
+/*
+ * Which matrices the components are solved in.  into[k] = { matrix, first row in it } of component k; the sizes of the
+ * matrices are returned.  Those of up to RMT_BLOCK rows run in k_rmt_blocks if `blocks` is set on return.
+ *
+ * Times of one threshold, in the 0.030 ms that the library's solver takes per row: a matrix of r rows max(r, r^2 / 1,700)
+ * there (64 rows 1.6 ms, 128 4.1, 200 6.0, 1,000 30, 3,000 159, 7,800 1,063), and k_rmt_blocks 1.5 per row of its largest
+ * component, whatever their number up to a wave (32 rows 1.3 ms, 64 2.6, 128 6.1; 10 of 128 6.2).  So
+ *  - one matrix of all rows where that is no slower than the parts: one component with two thirds of the rows or more
+ *    (a component of 64 rows alone: 2.6 -> 1.6 ms);
+ *  - else the components above RMT_BLOCK rows share matrices of about RMT_SHARED rows, up to which a row costs the same
+ *    and each solve by itself costs more (8 components of 129 rows: 34.5 -> 27.5 ms).
+ */
+constexpr double RMT_SHARED = 1280.0;
+
+static std::vector<int32_t> rmt_plan(const std::vector<int32_t>& size, int sms, std::vector<int2>& into, bool& blocks)
+{
+   auto solver = [](double r) { return std::max(r, r * r / 1700.0); };
+   double all = 0.0, large = 0.0;
+   int32_t most[2] = { 0, 0 };
+   int64_t count[2] = { 0, 0 };
+   for ( int32_t n : size )
+   {
+      all += n;
+      if ( n > RMT_BLOCK )
+         large += n;
+      else
+      {
+         const int wide = n > RMT_BLOCK_WARP;
+         most[wide] = std::max(most[wide], n);
+         ++count[wide];
+      }
+   }
+   const int groups = (int)std::ceil(large / RMT_SHARED);
+   const double target = groups > 0 ? large / groups : 0.0;
+   std::vector<int32_t> matrix;
+   into.assign(size.size(), make_int2(0, 0));
+   double parts = 0.0;
+   int shared = -1;                                      /* the matrix that large components are being added to */
+   for ( size_t k = 0; k < size.size(); ++k )
+   {
+      if ( size[k] <= RMT_BLOCK || shared < 0 || matrix[(size_t)shared] >= target )
+      {
+         into[k] = make_int2((int)matrix.size(), 0);
+         if ( size[k] > RMT_BLOCK ) shared = (int)matrix.size();
+         matrix.push_back(size[k]);
+      }
+      else
+      {
+         into[k] = make_int2(shared, matrix[(size_t)shared]);
+         matrix[(size_t)shared] += size[k];
+      }
+   }
+   for ( int32_t n : matrix )
+      if ( n > RMT_BLOCK ) parts += solver(n);
+   for ( int wide = 0; wide < 2; ++wide )
+   {
+      const double per_sm = std::min(32.0, std::floor(227.0 * 1024 / (double)(rmt_block_bytes(most[wide]) + 1024)));
+      parts += 1.5 * most[wide] * std::ceil((double)count[wide] / (per_sm * sms));
+   }
+   blocks = solver(all) > parts;
+   if ( !blocks )
+   {
+      int32_t at = 0;
+      for ( size_t k = 0; k < size.size(); ++k )
+      {
+         into[k] = make_int2(0, at);
+         at += size[k];
+      }
+      matrix.assign(1, at);
+   }
+   return matrix;
+}
+
+/* the eigenvalues of one matrix by the library: from dA + at into dW + values */
+int large_matrix(RmtDevice& d, const RmtComponent& q)
 {
    if ( !d.solver && (cusolverDnCreate(&d.solver) != CUSOLVER_STATUS_SUCCESS
                       || cusolverDnSetStream(d.solver, d.st) != CUSOLVER_STATUS_SUCCESS) )
@@ -420,8 +498,7 @@ int device_eigenvalues(RmtDevice& d, float t, std::vector<float>& eig, int32_t& 
    /* the components in the order of their first rows, and each row's place */
    eig.clear();
    m = 0;
-   std::vector<RmtComponent> comp;
-   std::vector<int32_t> list[2];                         /* blocks for a warp, and for a larger CTA */
+   std::vector<int32_t> size;
    for ( int64_t i = 0; i < rows; ++i )
    {
       const int32_t root = d.root[(size_t)i];
@@ -430,12 +507,12 @@ int device_eigenvalues(RmtDevice& d, float t, std::vector<float>& eig, int32_t& 
       {
          if ( root == i )
          {
-            p.x = (int)comp.size();
-            comp.push_back(RmtComponent { 0, 0, 0 });
+            p.x = (int)size.size();
+            size.push_back(0);
          }
          else
             p.x = d.place[(size_t)root].x;               /* a root is its component's first row */
-         p.y = comp[(size_t)p.x].size++;
+         p.y = size[(size_t)p.x]++;
          ++m;
       }
       d.place[(size_t)i] = p;
@@ -449,20 +526,27 @@ int device_eigenvalues(RmtDevice& d, float t, std::vector<float>& eig, int32_t& 
       eig.assign((size_t)m, std::numeric_limits<float>::quiet_NaN());
       return KINC_SIM_OK;
    }
+   std::vector<int2> into;
+   bool blocks = true;
+   const std::vector<int32_t> matrix = rmt_plan(size, d.sms, into, blocks);
+   if ( matrix.size() != size.size() )
+      for ( int2& p : d.place )
+         if ( p.x >= 0 ) p = make_int2(into[(size_t)p.x].x, into[(size_t)p.x].y + p.y);
+   auto in_block = [&](int32_t n) { return blocks && n <= RMT_BLOCK; };
    size_t need = 0;
    int32_t values = 0, most[2] = { 0, 0 };
-   for ( size_t k = 0; k < comp.size(); ++k )
+   std::vector<RmtComponent> comp;
+   std::vector<int32_t> list[2];                         /* blocks for a warp, and for a larger CTA */
+   for ( int32_t n : matrix )
    {
-      RmtComponent& q = comp[k];
-      if ( q.size > RMT_BLOCK ) need = (need + 31) & ~(size_t)31;      /* the library's matrices on 256-byte boundaries */
-      q.at = (int64_t)need;
-      q.values = values;
-      need += (size_t)q.size * q.size;
-      values += q.size;
-      if ( q.size > RMT_BLOCK ) continue;
-      const int wide = q.size > RMT_BLOCK_WARP;
-      list[wide].push_back((int32_t)k);
-      most[wide] = std::max(most[wide], q.size);
+      if ( !in_block(n) ) need = (need + 31) & ~(size_t)31;      /* the library's matrices on 256-byte boundaries */
+      comp.push_back(RmtComponent { (int64_t)need, n, values });
+      need += (size_t)n * n;
+      values += n;
+      if ( !in_block(n) ) continue;
+      const int wide = n > RMT_BLOCK_WARP;
+      list[wide].push_back((int32_t)comp.size() - 1);
+      most[wide] = std::max(most[wide], n);
    }
    if ( need > d.capA )
    {
@@ -492,8 +576,8 @@ int device_eigenvalues(RmtDevice& d, float t, std::vector<float>& eig, int32_t& 
    }
    for ( const RmtComponent& q : comp )
    {
-      if ( q.size <= RMT_BLOCK ) continue;
-      const int rc = large_component(d, q);
+      if ( in_block(q.size) ) continue;
+      const int rc = large_matrix(d, q);
       if ( rc ) return rc;
    }
    std::vector<double> w((size_t)m);

@@ -96,3 +96,10 @@ def test_infinite_items_have_no_eigenvalues(rows, a, b, value):
     threshold, steps = RMT(tstart=0.7, tstep=0.05, tstop=0.5).run(items=(x, y, c, r), genes=G + rows, max_clusters=1,
                                                                   strict=False)
     assert threshold is None and len(steps) >= 4 and np.all(steps[:, 2] == -1.0)
+
+
+@pytest.mark.parametrize("groups", [[90, 20], [64], [20, 3], [129] * 8, [130] * 11 + [40, 3, 2], [900, 140, 700, 129, 5]])
+def test_components_that_share_a_matrix(groups):
+    """One component with most of the rows, and components above the block solver's limit: solved in matrices that
+    hold several of them."""
+    _check(*(lambda n: (n[0], 1) + n[1:])(_network(groups, "chain", seed=8)), 0.6)
