@@ -633,6 +633,22 @@ static size_t warp_smem(const SimKernel& k, size_t sort_bytes)
    return k.clus == 2 && k.ks > 0 ? std::max(sort_bytes, (size_t)KM_RING_BYTES) : sort_bytes;
 }
 
+/*
+ * Lets a kernel be launched with all the dynamic shared memory a CTA can have.  The limit belongs to the kernel on
+ * its device, not to a context: a context that lowered it to its own need would take the launches from the contexts
+ * (and threads) that need more, so every caller sets the same one.
+ */
+static cudaError_t allow_shared_memory(const void* fn)
+{
+   int dev = 0, optin = 0;
+   cudaFuncAttributes a {};
+   cudaError_t e = cudaGetDevice(&dev);
+   if ( e == cudaSuccess ) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+   if ( e == cudaSuccess ) e = cudaFuncGetAttributes(&a, fn);
+   if ( e != cudaSuccess ) return e;
+   return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes);
+}
+
 /* the shape measured best on the clustering workloads: CTAs of the kernel's full warp count (20
  * for GMM, 16 otherwise), rounds for GMM and no clustering, free-running warps for K-means, the
  * sweeps prefetching 8 samples ahead */
@@ -776,9 +792,7 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
    ctx->smem_warp = (int)(warp_smem(ctx->kern, ctx->smem_sort ? sort_bytes_warp : 0) + param_bytes_warp);
    dp.smem_floats = ctx->smem_warp / (int)sizeof(float);
    ctx->smem_bytes = ctx->smem_warp * wpb;
-   /* opt in whenever dynamic shared memory is used: the kernel's own static words count against 48 KB too */
-   if ( ctx->smem_bytes > 0 )
-      CKC(cudaFuncSetAttribute(ctx->kern.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->smem_bytes));
+   CKC(allow_shared_memory(ctx->kern.fn));
    int per_sm = 0;
    CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ctx->kern.fn, wpb * 32, ctx->smem_bytes));
    per_sm = std::max(1, per_sm);
@@ -1649,8 +1663,7 @@ extern "C" int kinc_sim_execute_block_noalloc(const float* d_gem, int32_t genes,
    const int smem_warp = (int)(warp_smem(kern, smem_sort ? sort_bytes_warp : 0) + param_bytes_warp);
    dp.smem_floats = smem_warp / (int)sizeof(float);
    const int smem_bytes = smem_warp * wpb;
-   if ( smem_bytes > 0 )
-      CK(cudaFuncSetAttribute(kern.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+   CK(allow_shared_memory(kern.fn));
 
    /* carve the static array: fixed parts first, then as many warp slots as fit */
    size_t off = 0;

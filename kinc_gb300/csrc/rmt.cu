@@ -569,7 +569,8 @@ int device_eigenvalues(RmtDevice& d, float t, std::vector<float>& eig, int32_t& 
       if ( count == 0 ) continue;
       const int smem = (int)rmt_block_bytes(most[wide]);
       RCK(cudaMemcpyAsync(to, list[wide].data(), (size_t)count * sizeof(int32_t), cudaMemcpyHostToDevice, d.st));
-      RCK(cudaFuncSetAttribute(k_rmt_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      /* the kernel's limit, the same for every caller (it belongs to the kernel, not to a call) */
+      RCK(cudaFuncSetAttribute(k_rmt_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rmt_block_bytes(RMT_BLOCK)));
       k_rmt_blocks<<<count, wide ? RMT_BLOCK : RMT_BLOCK_WARP, smem, d.st>>>(d.dcomp, to, count, d.dA, d.dW);
       RCK(cudaGetLastError());
       to += count;

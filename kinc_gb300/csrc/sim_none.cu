@@ -144,6 +144,8 @@ static cudaError_t sim_launch_pearson_lanes(int sms, cudaStream_t st, const DevP
  */
 constexpr int PT_THREADS = 128;
 constexpr int PT_WORDS = 128;
+constexpr int PT_SMEM = 100 * 1024;         /* dynamic shared memory at most; the kernels' limit, the same for every caller
+                                               (it belongs to the kernel, not to a context) */
 
 /* a tile of TX x (512 / TX) genes; few rows x take flat tiles */
 template <int TX>
@@ -357,7 +359,7 @@ static cudaError_t launch_pearson_tiles(cudaStream_t st, const DevParams& P, con
                                         int x1)
 {
    const int smem = (int)PearsonTile<TX>::bytes(P.W);
-   const cudaError_t e = cudaFuncSetAttribute(k_pearson_tiles<TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+   const cudaError_t e = cudaFuncSetAttribute(k_pearson_tiles<TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM);
    if ( e != cudaSuccess ) return e;
    const dim3 grid((x1 + PearsonTile<TX>::Y - 1) / PearsonTile<TX>::Y, (x1 - x0) / TX + 1);
    k_pearson_tiles<TX><<<grid, PT_THREADS, smem, st>>>(P, D, B, x0);
@@ -375,8 +377,8 @@ cudaError_t sim_launch_pearson(int sms, cudaStream_t st, const DevParams& P, con
    };
    const int x0 = row_of(B.start), x1 = row_of(B.start + B.size - 1), rows = x1 - x0 + 1;
    /* the masks of a tile's genes lie in shared memory beside 32 samples of their values */
-   if ( rows <= 2 && PearsonTile<2>::bytes(P.W) <= 100 * 1024 ) return launch_pearson_tiles<2>(st, P, D, B, x0, x1);
-   if ( rows <= 8 && PearsonTile<4>::bytes(P.W) <= 100 * 1024 ) return launch_pearson_tiles<4>(st, P, D, B, x0, x1);
+   if ( rows <= 2 && PearsonTile<2>::bytes(P.W) <= PT_SMEM ) return launch_pearson_tiles<2>(st, P, D, B, x0, x1);
+   if ( rows <= 8 && PearsonTile<4>::bytes(P.W) <= PT_SMEM ) return launch_pearson_tiles<4>(st, P, D, B, x0, x1);
    if ( P.W <= PT_WORDS ) return launch_pearson_tiles<16>(st, P, D, B, x0, x1);
    return sim_launch_pearson_lanes(sms, st, P, D, B);
 }
@@ -398,6 +400,11 @@ constexpr int ORDER_THREADS = 256;
 constexpr int ORDER_MOST = 8192;            /* samples k_gene_order sorts in shared memory (64 KB of keys) */
 constexpr uint16_t ORDER_TIE = 0x8000;
 constexpr int SPEARMAN_WARPS = 8;
+/* dynamic shared memory at ORDER_MOST samples: the kernels' limits, the same for every caller (they belong to the
+ * kernels, not to a context) */
+constexpr int ORDER_SMEM = ORDER_MOST * (int)sizeof(unsigned long long);
+constexpr int SPEARMAN_SMEM = SPEARMAN_WARPS * (ORDER_MOST / 8 + ORDER_MOST * (int)sizeof(uint16_t));
+constexpr int TIES_SMEM = ORDER_MOST / 8 + 2 * ORDER_MOST * (int)sizeof(float);
 
 /* order[g][r]: the r-th of gene g's usable samples by value, ORDER_TIE set if the next one is equal; filled up
  * with samples the gene lacks.  ties[g]: 1 if any is set, 2 added if the gene has +inf, with which the network
@@ -468,7 +475,7 @@ size_t sim_spearman_orders_bytes(const DevParams& P, char* base, SpearmanOrders*
 cudaError_t sim_spearman_orders(cudaStream_t st, const DevParams& P, const DevData& D, const SpearmanOrders& R)
 {
    const int smem = P.P2 * (int)sizeof(unsigned long long);
-   const cudaError_t e = cudaFuncSetAttribute(k_gene_order, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+   const cudaError_t e = cudaFuncSetAttribute(k_gene_order, cudaFuncAttributeMaxDynamicSharedMemorySize, ORDER_SMEM);
    if ( e != cudaSuccess ) return e;
    k_gene_order<<<std::min(P.G, 16384), ORDER_THREADS, smem, st>>>(D.gem, D.umask, P.G, P.S, P.W, P.P2, R.order, R.ties);
    return cudaGetLastError();
@@ -639,8 +646,8 @@ cudaError_t sim_launch_spearman(int sms, cudaStream_t st, const DevParams& P, co
    const int bytes = mask + ((P.S * 2 + 15) & ~15);
    const int smem = bytes * SPEARMAN_WARPS, net = mask + 2 * P.P2 * (int)sizeof(float);
    int per_sm = 1, net_per_sm = 1;
-   cudaError_t e = cudaFuncSetAttribute(k_spearman_orders, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-   if ( e == cudaSuccess ) e = cudaFuncSetAttribute(k_spearman_ties, cudaFuncAttributeMaxDynamicSharedMemorySize, net);
+   cudaError_t e = cudaFuncSetAttribute(k_spearman_orders, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEARMAN_SMEM);
+   if ( e == cudaSuccess ) e = cudaFuncSetAttribute(k_spearman_ties, cudaFuncAttributeMaxDynamicSharedMemorySize, TIES_SMEM);
    if ( e == cudaSuccess )
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spearman_orders, SPEARMAN_WARPS * 32, smem);
    if ( e == cudaSuccess ) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&net_per_sm, k_spearman_ties, 32, net);
