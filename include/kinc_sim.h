@@ -181,8 +181,21 @@ int kinc_sim_pair_counts(kinc_sim_ctx* ctx, int64_t start, int64_t size, int32_t
 /* Kernel launches made by the last kinc_sim_execute_block* call (for accounting). */
 int32_t kinc_sim_last_launch_count(const kinc_sim_ctx* ctx);
 
+/* What computed the pairs of the last kinc_sim_execute_block* call's last device block. */
+enum
+{
+   KINC_SIM_KERNEL_NONE = 0,          /* no block yet */
+   KINC_SIM_KERNEL_TILES = 1,         /* the tile kernel: 32 pairs per warp, one per lane */
+   KINC_SIM_KERNEL_GMM_PAIRS = 2,     /* GMM up to 5 clusters, one warp per pair */
+   KINC_SIM_KERNEL_KMEANS_PAIRS = 3,  /* K-means up to 5 clusters, a stream of pairs per warp */
+   KINC_SIM_KERNEL_GENES = 4,         /* no clustering: Pearson from the rows of the matrix, Spearman from the genes'
+                                         sample orders */
+   KINC_SIM_KERNEL_CONTRACTION = 5    /* precision 1 to 4 */
+};
+int32_t kinc_sim_last_kernel(const kinc_sim_ctx* ctx);
+
 /*
- * Launch shape of the per-pair kernel.  Every shape computes the same bits;
+ * Launch shape of the kernels that work in warp slots.  Every shape computes the same bits;
  * only the speed differs, so the shape is picked by measurement
  * (kinc_sim_autotune) rather than fixed.  Replaces the hand-set work-item
  * count of KINC's OpenCL worker (--ksize, src/core/similarity_input.cpp:241-251),
@@ -193,11 +206,11 @@ int32_t kinc_sim_last_launch_count(const kinc_sim_ctx* ctx);
  *                  round (they then run the same code region at the same time);
  *                  0: every warp takes its next tile as soon as it is done
  *   prefetch       0, 4, 8 or 16: samples ahead the GMM EM passes prefetch into L2
- * K-means up to 5 clusters takes only warps_per_cta (its warps work apart).
- * Pearson without clustering (clusmethod none, corrmethod pearson) runs one thread
- * per pair and takes no shape; neither do the blocks that run GMM with one warp per
- * pair (up to 5 clusters; blocks that do not fill the tile kernel's waves well enough
- * to make up for its slower samples).
+ * The tile kernel takes all three; K-means up to 5 clusters only warps_per_cta (its
+ * warps work apart).  The other kernels take none: GMM with one warp per pair (up to 5
+ * clusters; the blocks that do not fill the tile kernel's waves well enough), and
+ * without clustering Pearson and, up to 8,192 samples, Spearman
+ * (kinc_sim_last_kernel tells which one ran).
  */
 typedef struct kinc_sim_launch
 {
@@ -223,14 +236,18 @@ int kinc_sim_set_launch(kinc_sim_ctx* ctx, const kinc_sim_launch* launch);
  * capped at kinc_sim_max_device_block) run once per candidate on the context's
  * stream, timed with CUDA events, in a coordinate descent from the current
  * shape over prefetch (clustering only), warps_per_cta and rounds (not for GMM,
- * which keeps the current shape's rounds); the fastest is applied.  With use_cache, the shape is first looked up -- and afterwards
- * stored -- in a small text cache keyed by the clustering and correlation
- * arguments, max_clusters, the sample count rounded up to a power of two and
- * the GPU (file: $KINC_TUNE_CACHE, else $XDG_CACHE_HOME/kinc_gb300/launch.txt,
- * else ~/.cache/kinc_gb300/launch.txt); a cache hit times nothing.  Up to
- * `cap` timed candidates are written to `entries` (may be NULL) and their
- * count to *n.  Synchronises the context's stream; the per-pair outputs of the
- * timed runs are discarded.  Not available for the tensor-core precisions.
+ * which keeps the current shape's rounds; K-means up to 5 clusters: warps_per_cta
+ * only); the fastest is applied.  GMM times the tile kernel, whichever kernel a block
+ * of this size would run in; a context whose blocks never run there times one wave of
+ * it, in scratch that is freed again.  Where no kernel takes a shape nothing is timed
+ * or stored and *chosen is the current one.  With use_cache, the shape is first looked
+ * up -- and afterwards stored -- in a small text cache keyed by the kernel, the
+ * clustering and correlation arguments, max_clusters, the sample count rounded up to a
+ * power of two and the GPU (file: $KINC_TUNE_CACHE, else
+ * $XDG_CACHE_HOME/kinc_gb300/launch.txt, else ~/.cache/kinc_gb300/launch.txt); a cache
+ * hit times nothing.  Up to `cap` timed candidates are written to `entries` (may be
+ * NULL) and their count to *n.  Synchronises the context's stream; the per-pair outputs
+ * of the timed runs are discarded.  Not available for the tensor-core precisions.
  */
 int kinc_sim_autotune(kinc_sim_ctx* ctx, int64_t start, int64_t size, int32_t use_cache, kinc_sim_launch* chosen,
                       kinc_sim_tune_entry* entries, int32_t cap, int32_t* n);

@@ -394,6 +394,7 @@ struct kinc_sim_ctx
    /* host-side tracking of the rand() position held in d_qbase */
    int64_t q_valid_end = 0;
    int32_t launches = 0;
+   int32_t last_kernel = KINC_SIM_KERNEL_NONE;
    std::string err;
 };
 
@@ -577,6 +578,11 @@ extern "C" int32_t kinc_sim_last_launch_count(const kinc_sim_ctx* ctx)
    return ctx ? ctx->launches : 0;
 }
 
+extern "C" int32_t kinc_sim_last_kernel(const kinc_sim_ctx* ctx)
+{
+   return ctx ? ctx->last_kernel : KINC_SIM_KERNEL_NONE;
+}
+
 extern "C" int kinc_sim_work_counters(kinc_sim_ctx* ctx, uint64_t* out, int reset)
 {
    if ( !ctx || !out ) return KINC_SIM_EINVAL;
@@ -623,6 +629,56 @@ static KmPool km_pool_sizes(const kinc_sim_params& p, const SimKernel& k)
    m.bytes = (((size_t)m.dmax * TILE * sizeof(int32_t) + 255) & ~(size_t)255)
              + (((size_t)m.tmax * m.rs * sizeof(float) + 255) & ~(size_t)255);
    return m;
+}
+
+/* K-means with local-memory centroids (more than 5 clusters) reads a contiguous copy of the lane's samples */
+static bool lane_major(const kinc_sim_params& p, const SimKernel& k)
+{
+   return p.clus_method == 2 && KINC_KMEANS_LANE_MAJOR && k.ks == 0;
+}
+
+/* the scratch of the kernels that work in warp slots (32-pair tiles, and the K-means streams) */
+static cudaError_t tile_scratch(kinc_sim_ctx* ctx)
+{
+   const size_t slots = (size_t)ctx->slots, col = (size_t)ctx->S * TILE;
+   const KmPool km = km_pool_sizes(ctx->params, ctx->kern);
+   size_t off = 0;
+   auto take = [&](size_t bytes) {
+      const size_t o = off;
+      off += (bytes + 255) & ~(size_t)255;
+      return o;
+   };
+   const size_t oX = take(slots * col * sizeof(float2));
+   const size_t oL = take(slots * col * sizeof(float));
+   const size_t oG = take(slots * col * sizeof(float) * ctx->dp.gam_k);
+   const size_t oB = take(slots * col);
+   const size_t oW = take(slots * col);
+   const size_t oA = take(slots * col);
+   const size_t oY = take(slots * col);
+   const size_t oC = take(slots * col);
+   const size_t oR = take(slots * RNG_WORDS * TILE * sizeof(uint32_t));
+   const size_t oS = take(ctx->smem_sort ? 0 : slots * ctx->dp.sort_floats * sizeof(float));
+   const bool xl = lane_major(ctx->params, ctx->kern);
+   const size_t oXl = take(xl ? slots * col * sizeof(float2) : 0);
+   const size_t oKd = take(slots * (size_t)km.dmax * TILE * sizeof(int32_t));
+   const size_t oKr = take(slots * (size_t)km.tmax * km.rs * sizeof(float));
+   const cudaError_t e = cudaMalloc(&ctx->d_scratch, off);
+   if ( e != cudaSuccess ) return e;
+   char* base = (char*)ctx->d_scratch;
+   ctx->ds.X = (float2*)(base + oX);
+   ctx->ds.lpx = (float*)(base + oL);
+   ctx->ds.gam = ctx->dp.gam_k ? (float*)(base + oG) : nullptr;
+   ctx->ds.lbl = (int8_t*)(base + oB);
+   ctx->ds.wl = (int8_t*)(base + oW);
+   ctx->ds.ya = (int8_t*)(base + oA);
+   ctx->ds.yb = (int8_t*)(base + oY);
+   ctx->ds.yc = (int8_t*)(base + oC);
+   ctx->ds.rng = (uint32_t*)(base + oR);
+   ctx->ds.sortbuf = ctx->smem_sort ? nullptr : (float*)(base + oS);
+   ctx->ds.Xl = xl ? (float2*)(base + oXl) : nullptr;
+   ctx->ds.kmd = km.bytes ? (int32_t*)(base + oKd) : nullptr;
+   ctx->ds.kmr = km.bytes ? (float*)(base + oKr) : nullptr;
+   return cudaSuccess;
 }
 
 /* ---------------------------------------------------------- launch shape */
@@ -801,14 +857,10 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
    const size_t col = (size_t)S * TILE;
    dp.gam_k = (KINC_STORE_GAMMA && params->clus_method == 1)
                  ? (params->max_clusters <= 3 ? 3 : params->max_clusters <= 5 ? 5 : 0) : 0;
-   /* K-means with register-resident means (up to 3 or 5 clusters) runs the tile as a task pool
-    * (draws and task records per slot); beyond that, per-lane fits over a contiguous copy of the
-    * lane's samples */
    const KmPool km = km_pool_sizes(*params, ctx->kern);
    dp.km_dmax = km.dmax;
    dp.km_tmax = km.tmax;
-   const bool lane_major = params->clus_method == 2 && KINC_KMEANS_LANE_MAJOR && ctx->kern.ks == 0;
-   const size_t slot_bytes = col * sizeof(float2) * (lane_major ? 2 : 1) + col * sizeof(float) * (1 + dp.gam_k)
+   const size_t slot_bytes = col * sizeof(float2) * (lane_major(*params, ctx->kern) ? 2 : 1) + col * sizeof(float) * (1 + dp.gam_k)
                              + 5 * col + (size_t)RNG_WORDS * TILE * sizeof(uint32_t)
                              + (ctx->smem_sort ? 0 : sort_bytes_warp) + km.bytes + 256 * 10;
    size_t free_b = 0, total_b = 0;
@@ -851,43 +903,7 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
     * warp per pair; without clustering it is left with Spearman of more samples than the orders take) */
    const bool tiles = params->precision == 0 && (params->clus_method != 0 || (params->corr_method != 0 && !ctx->d_orders))
                       && !sim_gmm_pairs_better(ctx->gmm_per_sm, ctx->gmm_wave, ctx->gmm_wave);
-   if ( tiles )
-   {
-      size_t off = 0;
-      auto take = [&](size_t bytes) {
-         const size_t o = off;
-         off += (bytes + 255) & ~(size_t)255;
-         return o;
-      };
-      const size_t oX = take(slots * col * sizeof(float2));
-      const size_t oL = take(slots * col * sizeof(float));
-      const size_t oG = take(slots * col * sizeof(float) * dp.gam_k);
-      const size_t oB = take(slots * col);
-      const size_t oW = take(slots * col);
-      const size_t oA = take(slots * col);
-      const size_t oY = take(slots * col);
-      const size_t oC = take(slots * col);
-      const size_t oR = take(slots * RNG_WORDS * TILE * sizeof(uint32_t));
-      const size_t oS = take(ctx->smem_sort ? 0 : slots * sort_bytes_warp);
-      const size_t oXl = take(lane_major ? slots * col * sizeof(float2) : 0);
-      const size_t oKd = take(slots * (size_t)km.dmax * TILE * sizeof(int32_t));
-      const size_t oKr = take(slots * (size_t)km.tmax * km.rs * sizeof(float));
-      CKC(cudaMalloc(&ctx->d_scratch, off));
-      char* base = (char*)ctx->d_scratch;
-      ctx->ds.X = (float2*)(base + oX);
-      ctx->ds.lpx = (float*)(base + oL);
-      ctx->ds.gam = dp.gam_k ? (float*)(base + oG) : nullptr;
-      ctx->ds.lbl = (int8_t*)(base + oB);
-      ctx->ds.wl = (int8_t*)(base + oW);
-      ctx->ds.ya = (int8_t*)(base + oA);
-      ctx->ds.yb = (int8_t*)(base + oY);
-      ctx->ds.yc = (int8_t*)(base + oC);
-      ctx->ds.rng = (uint32_t*)(base + oR);
-      ctx->ds.sortbuf = ctx->smem_sort ? nullptr : (float*)(base + oS);
-      ctx->ds.Xl = lane_major ? (float2*)(base + oXl) : nullptr;
-      ctx->ds.kmd = km.bytes ? (int32_t*)(base + oKd) : nullptr;
-      ctx->ds.kmr = km.bytes ? (float*)(base + oKr) : nullptr;
-   }
+   if ( tiles ) CKC(tile_scratch(ctx));
 
    /* one device block of pairs (the tensor-core form writes no labels, so its blocks can be far larger) */
    const int64_t total = (int64_t)genes * (genes - 1) / 2;
@@ -954,9 +970,16 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
 #undef CKC
 }
 
-/* enqueue one device block [start, start+size) into device outputs */
+/* K-means with a stream of pairs per warp (up to 5 clusters) */
+static bool streams_pairs(const kinc_sim_ctx* ctx)
+{
+   return ctx->params.clus_method == 2 && ctx->kern.ks > 0;
+}
+
+/* enqueue one device block [start, start+size) into device outputs; in_tiles: GMM in the tile kernel, whatever the
+ * block's size */
 static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t* d_K, int8_t* d_labels,
-                         float* d_corr, cudaStream_t st)
+                         float* d_corr, cudaStream_t st, bool in_tiles = false)
 {
    const DevParams& dp = ctx->dp;
    if ( ctx->use_tc )
@@ -964,6 +987,7 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
       int launches = 0;
       CK(tc_enqueue(ctx->tc, ctx->G, ctx->S, dp.min_samples, dp.max_k, start, size, d_K, d_corr, ctx->d_status, st,
                     &launches));
+      ctx->last_kernel = KINC_SIM_KERNEL_CONTRACTION;
       ctx->launches += launches;
       return KINC_SIM_OK;
    }
@@ -1007,7 +1031,7 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
       CK(launch_links(ctx->d_N, ctx->d_most32, span, ctx->d_pg, st));
       ++launches;
    }
-   /* Pearson without clustering runs one thread per pair straight from the matrix (no tiles) */
+   /* Pearson without clustering, and Spearman from the genes' orders, run straight from the matrix */
    const bool lanes = dp.clus == 0 && (dp.corr == 0 || (dp.corr == 2 && orders));
    if ( ctx->d_order && size > TILE && !lanes && !orders )
    {
@@ -1034,6 +1058,7 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
    B.tiles = ctx->d_tiles;
    B.status = ctx->d_status;
    B.work = ctx->d_work;
+   ctx->last_kernel = KINC_SIM_KERNEL_GENES;
    if ( lanes )
    {
       CK(sim_launch_pearson(ctx->sms, st, dp, ctx->dd, B));
@@ -1048,12 +1073,15 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
       ++launches;
       CK(sim_launch_spearman(ctx->sms, st, dp, ctx->dd, B, ctx->orders, ctx->d_tied));
    }
-   else if ( sim_gmm_pairs_better(ctx->gmm_per_sm, size, ctx->gmm_wave) )
+   else if ( !in_tiles && sim_gmm_pairs_better(ctx->gmm_per_sm, size, ctx->gmm_wave) )
    {
+      ctx->last_kernel = KINC_SIM_KERNEL_GMM_PAIRS;
       CK(sim_launch_gmm_pairs(ctx->sms, st, dp, ctx->dd, ctx->dsp, B, ctx->n_cap));
    }
    else
    {
+      if ( !ctx->d_scratch ) return fail(ctx, KINC_SIM_ECUDA, "no scratch for a block of %lld pairs", (long long)size);
+      ctx->last_kernel = streams_pairs(ctx) ? KINC_SIM_KERNEL_KMEANS_PAIRS : KINC_SIM_KERNEL_TILES;
       const SimKernel& k = ctx->kern;
       cudaError_t e = k.clus == 0 ? sim_launch_none(k, ctx->grid, ctx->smem_bytes, st, dp, ctx->dd, ctx->ds, B,
                                                     ctx->smem_sort)
@@ -1145,8 +1173,8 @@ std::string tune_key(const kinc_sim_ctx* ctx)
 {
    const kinc_sim_params& p = ctx->params;
    char buf[400];
-   snprintf(buf, sizeof buf, "clus=%d ks=%d ocl=%d corr=%d sem=%d pre=%d post=%d maxk=%d S<=%d gpu=%s sms=%d",
-            p.clus_method, ctx->kern.ks, (int)ctx->kern.ocl, p.corr_method, p.semantics, p.pre_out, p.post_out,
+   snprintf(buf, sizeof buf, "kernel=%s clus=%d ks=%d ocl=%d corr=%d sem=%d pre=%d post=%d maxk=%d S<=%d gpu=%s sms=%d",
+            streams_pairs(ctx) ? "stream" : "tiles", p.clus_method, ctx->kern.ks, (int)ctx->kern.ocl, p.corr_method, p.semantics, p.pre_out, p.post_out,
             p.max_clusters, next_pow2_host(std::max(ctx->S, 2)), ctx->gpu_name, ctx->sms);
    for ( char* c = buf; *c; ++c )
       if ( *c == '\t' || *c == '\n' ) *c = ' ';
@@ -1206,7 +1234,7 @@ static int time_launch(kinc_sim_ctx* ctx, const kinc_sim_launch& l, int64_t star
    CK(cudaEventCreate(&e0));
    CK(cudaEventCreate(&e1));
    cudaError_t err = cudaEventRecord(e0, ctx->stream);
-   rc = err == cudaSuccess ? enqueue_block(ctx, start, size, ctx->d_K, ctx->d_labels, ctx->d_corr, ctx->stream)
+   rc = err == cudaSuccess ? enqueue_block(ctx, start, size, ctx->d_K, ctx->d_labels, ctx->d_corr, ctx->stream, true)
                            : KINC_SIM_ECUDA;
    if ( rc == KINC_SIM_OK ) err = cudaEventRecord(e1, ctx->stream);
    if ( rc == KINC_SIM_OK && err == cudaSuccess ) err = cudaEventSynchronize(e1);
@@ -1230,6 +1258,12 @@ extern "C" int kinc_sim_autotune(kinc_sim_ctx* ctx, int64_t start, int64_t size,
    if ( rc ) return rc;
    size = std::min(size, ctx->max_block);
    if ( size <= 0 ) return fail(ctx, KINC_SIM_EINVAL, "autotune needs at least one pair");
+   if ( ctx->params.clus_method == 0 && (ctx->params.corr_method == 0 || ctx->orders.order) )
+   {
+      /* no kernel of this worker takes a shape: nothing to time or to keep */
+      if ( chosen ) *chosen = ctx->launch;
+      return KINC_SIM_OK;
+   }
    const std::string key = tune_key(ctx);
    kinc_sim_launch best = ctx->launch;
    if ( use_cache && tune_cache_lookup(key, ctx->kern.wpb, best) )
@@ -1239,6 +1273,25 @@ extern "C" int kinc_sim_autotune(kinc_sim_ctx* ctx, int64_t start, int64_t size,
       return rc;
    }
    CK(cudaStreamSynchronize(ctx->stream));
+   /* GMM: what is timed is the tile kernel, which alone takes a shape; a worker whose blocks never run there gets its
+    * scratch for this call, and times one wave */
+   struct Scratch
+   {
+      kinc_sim_ctx* ctx = nullptr;
+      ~Scratch()
+      {
+         if ( !ctx ) return;
+         cudaFree(ctx->d_scratch);
+         ctx->d_scratch = nullptr;
+         ctx->ds = DevScratch {};
+      }
+   } borrowed;
+   if ( !ctx->d_scratch )
+   {
+      CK(tile_scratch(ctx));
+      borrowed.ctx = ctx;
+      size = std::min(size, ctx->gmm_wave);
+   }
    int32_t count = 0;
    auto record = [&](const kinc_sim_launch& l, double ms) {
       if ( entries && count < cap ) entries[count] = kinc_sim_tune_entry { l, ms };
@@ -1253,7 +1306,8 @@ extern "C" int kinc_sim_autotune(kinc_sim_ctx* ctx, int64_t start, int64_t size,
    record(best, best_ms);
    const int warps_v[] = { 4, 8, 10, 16, 20 };
    const int pf_v[] = { 0, 4, 8, 16 };
-   for ( int pass = 0; pass < 2; ++pass )
+   const int passes = streams_pairs(ctx) ? 1 : 2;         /* one knob: one pass has timed all there is */
+   for ( int pass = 0; pass < passes; ++pass )
    {
       const kinc_sim_launch start_best = best;
       for ( int knob = 0; knob < 3; ++knob )
@@ -1264,6 +1318,7 @@ extern "C" int kinc_sim_autotune(kinc_sim_ctx* ctx, int64_t start, int64_t size,
           * 20 free-running warps from a 311,296-pair sample ran 1,048,576-pair blocks at 96k
           * pairs/s against 164k in rounds) */
          if ( knob == 2 && ctx->params.clus_method == 1 ) continue;
+         if ( knob != 1 && streams_pairs(ctx) ) continue;             /* its warps work apart and prefetch by their ring */
          const int nv = knob == 0 ? 4 : knob == 1 ? 5 : 2;
          const kinc_sim_launch base = best;
          for ( int v = 0; v < nv; ++v )

@@ -22,6 +22,7 @@ CRITERION_NAMES = ["BIC", "ICL"]
 SEMANTICS_NAMES = ["reference", "fixed"]
 RAND_NAMES = ["glibc", "lcg"]
 PRECISION_NAMES = ["fp32", "tf32", "3xbf16", "fp32tiled", "fp16"]
+KERNEL_NAMES = ["none", "tiles", "gmm pairs", "kmeans pairs", "genes", "contraction"]
 
 
 class InvalidArgument(ValueError):
@@ -202,6 +203,12 @@ class Similarity:
                                           entries, cap, ctypes.byref(n)), self._ctx)
         timed = [dict(entries[i].launch.as_dict(), ms=entries[i].ms) for i in range(min(n.value, cap))]
         return chosen.as_dict(), timed
+
+    def last_kernel(self):
+        """What computed the last block's pairs (kinc_sim_last_kernel)."""
+        if self._ctx is None:
+            return "none"
+        return KERNEL_NAMES[_native.load().kinc_sim_last_kernel(self._ctx)]
 
     def close(self):
         if self._ctx is not None:

@@ -63,3 +63,68 @@ def test_autotune_picks_a_timed_candidate_and_caches_it(tmp_path, monkeypatch):
     assert again == chosen and timed2 == []
     assert (tmp_path / "launch.txt").read_text().count("\t") == 2
     sim.close()
+
+
+def _wave():
+    """Pairs the GMM tile kernel runs at once: 20 warps of 32 on every SM."""
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count * 20 * 32
+
+
+def test_every_launch_shape_of_the_gmm_tile_kernel_gives_the_same_bits():
+    """A block of one full wave with two genes of many samples runs in tiles, one of a part of a wave does not."""
+    genes = 480
+    gem = synthetic.generate(2, genes=genes, samples=2600)
+    gem[:, 300:] = np.nan
+    gem[:2] = synthetic.generate(2, genes=2, samples=2600, seed=5)
+    sim = Similarity(gem, clusmethod="gmm", corrmethod="spearman", crit="BIC", maxclus=2, preout=True)
+    sim.initialize()
+    assert _wave() <= genes * (genes - 1) // 2
+    want = sim.execute(None, start=0, size=3000)
+    assert sim.last_kernel() == "gmm pairs"
+    for shape in SHAPES["gmm"]:
+        sim.set_launch(*shape)
+        got = sim.execute(None, start=0, size=_wave())
+        assert sim.last_kernel() == "tiles"
+        assert np.array_equal(got.K[:3000], want.K)
+        assert np.array_equal(got.labels[:3000][want.K > 1], want.labels[want.K > 1])
+        assert np.array_equal(got.corr[:3000], want.corr, equal_nan=True)
+    sim.close()
+
+
+def test_autotune_times_the_kernel_that_takes_the_shape(tmp_path, monkeypatch):
+    cache = tmp_path / "launch.txt"
+    monkeypatch.setenv("KINC_TUNE_CACHE", str(cache))
+    # GMM: the tile kernel, also where this worker's blocks run with one warp per pair
+    sim = Similarity(synthetic.generate(2, genes=40, samples=600), clusmethod="gmm", corrmethod="spearman", maxclus=2)
+    before = sim.execute(None, start=0, size=sim.total_pairs())
+    assert sim.last_kernel() == "gmm pairs"
+    _, timed = sim.autotune()
+    assert sim.last_kernel() == "tiles" and len(timed) >= 4
+    after = sim.execute(None, start=0, size=sim.total_pairs())
+    assert sim.last_kernel() == "gmm pairs"
+    assert np.array_equal(before.K, after.K) and np.array_equal(before.corr, after.corr, equal_nan=True)
+    sim.close()
+    assert cache.read_text().startswith("kernel=tiles ")
+    # K-means with a stream of pairs: warps per CTA only
+    sim = Similarity(synthetic.generate(4, genes=40, samples=80), clusmethod="kmeans", maxclus=3)
+    default = sim.launch()
+    _, timed = sim.autotune()
+    assert sim.last_kernel() == "kmeans pairs"
+    assert sorted(t["warps_per_cta"] for t in timed) == [4, 8, 16]
+    assert all(t[k] == default[k] for t in timed for k in ("rounds", "prefetch"))
+    sim.close()
+    assert cache.read_text().count("kernel=stream ") == 1
+
+
+@pytest.mark.parametrize("corr", ["pearson", "spearman", "both"])
+def test_autotune_without_a_shape_to_pick(corr, tmp_path, monkeypatch):
+    """Without clustering no kernel takes a shape: nothing is timed, and nothing is kept for other matrices."""
+    cache = tmp_path / "launch.txt"
+    monkeypatch.setenv("KINC_TUNE_CACHE", str(cache))
+    sim = Similarity(synthetic.generate(1, genes=50, samples=90), corrmethod=corr)
+    chosen, timed = sim.autotune()
+    assert chosen == sim.launch() and timed == [] and not cache.exists()
+    sim.execute(None, start=0, size=sim.total_pairs())
+    assert sim.last_kernel() == "genes"
+    sim.close()
