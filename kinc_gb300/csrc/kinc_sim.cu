@@ -88,6 +88,16 @@ __global__ void k_most_usable(const uint32_t* __restrict__ umask, int32_t G, int
    if ( lane == 0 ) atomicMax(most, best);
 }
 
+/* how many genes have each sample (count: W * 32); the mean N of all pairs is the sum of (count / G)^2 */
+__global__ void k_sample_genes(const uint32_t* __restrict__ umask, int32_t G, int32_t W, int* __restrict__ count)
+{
+   const int lane = threadIdx.x & 31, warps = (int)(blockDim.x >> 5), w = blockIdx.x;
+   int n = 0;
+   for ( int g = (int)blockIdx.y * warps + (int)(threadIdx.x >> 5); g < G; g += (int)gridDim.y * warps )
+      n += (int)((umask[(size_t)g * W + w] >> lane) & 1u);
+   atomicAdd(&count[w * 32 + lane], n);
+}
+
 __device__ __forceinline__ int pair_count(const uint32_t* __restrict__ umask, int W, int64_t p)
 {
    int32_t x, y;
@@ -358,6 +368,7 @@ struct kinc_sim_ctx
    int sms = 0;
    int64_t slots = 0;               /* warp scratch slots allocated */
    int n_cap = 0;                   /* no pair has more usable samples */
+   double n_mean = 0;               /* a pair's usable samples, on average */
    int gmm_per_sm = 0;              /* GMM with one warp per pair (sim_gmm_pair.cuh): pairs an SM holds, 0: not available */
    int64_t gmm_wave = 0;            /* pairs the tile kernel runs at once */
    DevScratch dsp {};               /* its scratch */
@@ -637,6 +648,12 @@ static bool lane_major(const kinc_sim_params& p, const SimKernel& k)
    return p.clus_method == 2 && KINC_KMEANS_LANE_MAJOR && k.ks == 0;
 }
 
+/* whether a block of `size` pairs runs GMM with one warp per pair */
+static bool gmm_in_pairs(const kinc_sim_ctx* ctx, int64_t size)
+{
+   return sim_gmm_pairs_better(ctx->dp, ctx->gmm_per_sm, ctx->n_mean, size, ctx->gmm_wave);
+}
+
 /* the scratch of the kernels that work in warp slots (32-pair tiles, and the K-means streams) */
 static cudaError_t tile_scratch(kinc_sim_ctx* ctx)
 {
@@ -871,15 +888,24 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
       grid -= prop.multiProcessorCount;
    const size_t slots = (size_t)grid * wpb;
    ctx->sms = prop.multiProcessorCount;
-   CKC(cudaMalloc(&ctx->d_status, sizeof(int)));
    ctx->n_cap = S;
    if ( params->clus_method == 1 )
    {
-      CKC(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
-      k_most_usable<<<std::min((genes + 7) / 8, 1024), 256, 0, ctx->stream>>>(ctx->d_umask, genes, W, ctx->d_status);
+      /* usable counts: genes of every sample, and the largest of a gene */
+      std::vector<int> usable((size_t)W * 32 + 1);
+      CKC(cudaMalloc(&ctx->d_order, usable.size() * sizeof(int)));
+      CKC(cudaMemsetAsync(ctx->d_order, 0, usable.size() * sizeof(int), ctx->stream));
+      k_sample_genes<<<dim3((unsigned)W, (unsigned)std::min((genes + 255) / 256, 64)), 256, 0, ctx->stream>>>(
+         ctx->d_umask, genes, W, ctx->d_order);
+      k_most_usable<<<std::min((genes + 7) / 8, 1024), 256, 0, ctx->stream>>>(ctx->d_umask, genes, W,
+                                                                              ctx->d_order + (size_t)W * 32);
       CKC(cudaGetLastError());
-      CKC(cudaMemcpyAsync(&ctx->n_cap, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      CKC(cudaMemcpyAsync(usable.data(), ctx->d_order, usable.size() * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
       CKC(cudaStreamSynchronize(ctx->stream));
+      CKC(cudaFree(ctx->d_order));
+      ctx->d_order = nullptr;
+      ctx->n_cap = usable.back();
+      for ( int i = 0; i < S; ++i ) ctx->n_mean += std::pow((double)usable[(size_t)i] / genes, 2.0);
       ctx->gmm_per_sm = sim_gmm_pairs_per_sm(dp, ctx->n_cap);
       ctx->gmm_wave = (int64_t)slots * TILE;
    }
@@ -899,18 +925,25 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
       dd.umask = ctx->d_umask;
       CKC(sim_spearman_orders(ctx->stream, dp, dd, ctx->orders));
    }
-   /* the tile kernel's scratch, where a block may run there (a whole wave is its best case against GMM with one
-    * warp per pair; without clustering it is left with Spearman of more samples than the orders take) */
-   const bool tiles = params->precision == 0 && (params->clus_method != 0 || (params->corr_method != 0 && !ctx->d_orders))
-                      && !sim_gmm_pairs_better(ctx->gmm_per_sm, ctx->gmm_wave, ctx->gmm_wave);
-   if ( tiles ) CKC(tile_scratch(ctx));
-
    /* one device block of pairs (the tensor-core form writes no labels, so its blocks can be far larger) */
    const int64_t total = (int64_t)genes * (genes - 1) / 2;
    int64_t mb = (int64_t)1 << 22;
    while ( mb > 4096 && (size_t)mb * S > ((size_t)1 << 31) ) mb >>= 1;
    if ( params->precision != 0 ) mb = (int64_t)1 << 27;
    ctx->max_block = std::min<int64_t>(mb, std::max<int64_t>(total, 1));
+
+   /* the tile kernel's scratch, where a block may run there (full waves, and the largest block, are its best case
+    * against GMM with one warp per pair; without clustering it is left with Spearman of more samples than the orders
+    * take) */
+   bool tiles = params->precision == 0 && (params->clus_method != 0 || (params->corr_method != 0 && !ctx->d_orders));
+   if ( tiles && ctx->gmm_per_sm > 0 )
+   {
+      tiles = !gmm_in_pairs(ctx, ctx->max_block);
+      for ( int64_t size = ctx->gmm_wave; size <= ctx->max_block && !tiles; size += ctx->gmm_wave )
+         tiles = !gmm_in_pairs(ctx, size);
+   }
+   if ( tiles ) CKC(tile_scratch(ctx));
+
    const int64_t nspan = (params->precision != 0 ? 4096 : ctx->max_block) + KINC_SIM_WORK_BLOCK_SIZE;
    const int64_t nscan = (ctx->max_block + SCAN_THREADS - 1) / SCAN_THREADS;
    CKC(cudaMalloc(&ctx->d_N, nspan * sizeof(int32_t)));
@@ -933,6 +966,7 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
    }
    if ( ctx->d_orders ) CKC(cudaMalloc(&ctx->d_tied, ctx->max_block * sizeof(int32_t)));
    CKC(cudaMemsetAsync(ctx->d_work, 0, 4 * sizeof(unsigned long long), ctx->stream));
+   CKC(cudaMalloc(&ctx->d_status, sizeof(int)));
    CKC(cudaMalloc(&ctx->d_K, ctx->max_block));
    if ( params->precision == 0 ) CKC(cudaMalloc(&ctx->d_labels, (size_t)ctx->max_block * S));
    CKC(cudaMalloc(&ctx->d_corr, (size_t)ctx->max_block * params->max_clusters * dp.ncorr * sizeof(float)));
@@ -1073,7 +1107,7 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
       ++launches;
       CK(sim_launch_spearman(ctx->sms, st, dp, ctx->dd, B, ctx->orders, ctx->d_tied));
    }
-   else if ( !in_tiles && sim_gmm_pairs_better(ctx->gmm_per_sm, size, ctx->gmm_wave) )
+   else if ( !in_tiles && gmm_in_pairs(ctx, size) )
    {
       ctx->last_kernel = KINC_SIM_KERNEL_GMM_PAIRS;
       CK(sim_launch_gmm_pairs(ctx->sms, st, dp, ctx->dd, ctx->dsp, B, ctx->n_cap));

@@ -18,17 +18,43 @@ int sim_gmm_pairs_per_sm(const DevParams& P, int n_cap)
 }
 
 /*
- * The tile kernel (one pair per lane) runs whole waves of `wave` pairs, however few there are; this one
- * takes pairs one by one.  Their rates at full waves, 97,280 pairs of the 10 %-missing mixture workload,
- * this kernel / the tile kernel, by pairs that fit an SM: 11 (N = 810) 187k / 168k per second, 10
- * (N = 1,134) 127k / 118k, 7 (N = 1,620) 81k / 87k, 4 (N = 2,430) 38k / 56k -- about 0.35 + 0.083 per
- * pair.  The tile kernel is taken where its wave is fuller than that.
+ * The tile kernel (one pair per lane) runs whole waves of `wave` pairs, however few there are, and its first wave
+ * takes a little longer (10 / n of one, n the usable samples of a pair); this one takes pairs one by one.  It is
+ * taken where the block's pairs, in waves, are no more than `rate` times the tile kernel's waves, rate being its own
+ * speed against the tile kernel's in full waves: the smaller of two.
+ *
+ *  - Few samples: the updates between the iterations (123 in units of the tile kernel's sample and component) and
+ *    what a sample takes besides its components outweigh the tile kernel's k n.  Measured / this formula, blocks of
+ *    389,120 pairs, Pearson: k <= 2 n = 40: 0.51 / 0.51, 97: 0.79 / 0.80, 243: 1.08 / 1.11; k <= 3 n = 63:
+ *    0.69 / 0.71; k <= 5 n = 40: 0.65 / 0.67, 63: 0.88 / 0.84, 97: 1.04 / 1.00, 162: 1.18 / 1.16.  One cluster
+ *    takes two iterations, so the pair's other work decides: n = 40: 0.39 (with outliers and Spearman 0.67), 97:
+ *    0.52 (0.88), 243: 0.79 (1.29), 810: 0.93 (1.60), and without sorts at most 0.84 in ten waves.
+ *  - Many samples: fewer pairs fit an SM.  97,280 pairs of the 10 %-missing mixture workload, k <= 5, Spearman with
+ *    outliers, by pairs that fit: 11 (N = 810) 187k / 168k per second, 8 (N = 1,215) 119k / 113k, 7 (N = 1,620)
+ *    81k / 87k, 4 (N = 2,430) 38k / 56k -- about 0.35 + 0.083 per pair.
  */
-bool sim_gmm_pairs_better(int per_sm, int64_t size, int64_t wave)
+bool sim_gmm_pairs_better(const DevParams& P, int per_sm, double n, int64_t size, int64_t wave)
 {
    if ( per_sm < 1 ) return false;
-   const double full = (double)size / (double)((size + wave - 1) / wave * wave);
-   return full <= 0.35 + 0.083 * per_sm;
+   n = std::max(n, 1.0);
+   double rate;
+   if ( P.max_k == 1 )
+   {
+      rate = gp_sort_rows(P) > 0 ? n / (0.75 * n + 38.0) : std::min(0.82, n / (n + 85.0));
+   }
+   else
+   {
+      double tiles = 0.0, here = 0.0;
+      for ( int k = std::max(P.min_k, 2); k <= P.max_k; ++k )
+      {
+         tiles += k * n;
+         here += 123.0 + n * (0.16 + 0.62 * k);
+      }
+      rate = tiles / here;
+   }
+   rate = std::min(rate, 0.35 + 0.083 * per_sm);
+   const double waves = (double)((size + wave - 1) / wave);
+   return (double)size / (double)wave <= rate * (waves + 10.0 / n);
 }
 
 size_t sim_gmm_pairs_scratch(int sms, const DevParams& P, int n_cap, char* base, DevScratch& W)

@@ -477,11 +477,11 @@ cudaError_t sim_kernel_launch_any(const SimKernel& k, int grid, int smem, cudaSt
                                   const DevData& D, const DevScratch& W, const DevBlock& B, int smem_sort);
 SimKernel sim_kernel_none();
 /* GMM with one warp per pair (sim_gmm_pair.cu): pairs an SM holds when no pair has more than n_cap usable
- * samples (0: these arguments do not run there), whether a block of `size` pairs runs faster there than in
- * the tile kernel's waves of `wave` pairs, the scratch (labels and responsibilities of the pairs in
+ * samples (0: these arguments do not run there), whether a block of `size` pairs with n usable samples on
+ * average runs faster there than in the tile kernel's waves of `wave` pairs, the scratch (labels and responsibilities of the pairs in
  * flight: returns the bytes, and sets W's pointers from base), and the launch */
 int sim_gmm_pairs_per_sm(const DevParams& P, int n_cap);
-bool sim_gmm_pairs_better(int per_sm, int64_t size, int64_t wave);
+bool sim_gmm_pairs_better(const DevParams& P, int per_sm, double n, int64_t size, int64_t wave);
 size_t sim_gmm_pairs_scratch(int sms, const DevParams& P, int n_cap, char* base, DevScratch& W);
 cudaError_t sim_launch_gmm_pairs(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevScratch& W,
                                  const DevBlock& B, int n_cap);

@@ -90,3 +90,46 @@ def test_block_that_fills_the_tile_kernel_s_wave():
     multi = part.K > 1
     assert np.array_equal(whole.labels[:5000][multi], part.labels[multi])
     assert np.array_equal(np.nan_to_num(whole.corr[:5000], nan=9.0), np.nan_to_num(part.corr, nan=9.0))
+
+
+def _slices(gem, gargs, oargs, start, size, slices):
+    """The block on the GPU; the oracle on parts of it.  Returns the kernel that ran and the result."""
+    sim = Similarity(gem, clusmethod="gmm", **gargs)
+    res = sim.execute(None, start=start, size=size)
+    kernel = sim.last_kernel()
+    sim.close()
+    for at, n in slices:
+        K, labels, corr, _ = pyoracle.run_block(gem, pyoracle.params(clus_method=1, **oargs), start + at, n)
+        got = slice(at, at + n)
+        assert np.array_equal(res.K[got], K)
+        assert np.array_equal(res.labels[got][K > 1], labels[K > 1])
+        assert np.array_equal(res.corr[got], corr, equal_nan=True)
+    return kernel, res
+
+
+@pytest.mark.parametrize("samples,gargs,oargs", [
+    (36, dict(maxclus=1, corrmethod="pearson", crit="BIC"), dict(max_clusters=1, corr_method=0, criterion=0)),
+    (50, dict(maxclus=2, corrmethod="spearman", crit="BIC", preout=True),
+     dict(max_clusters=2, corr_method=1, criterion=0, pre_out=1)),
+    (64, dict(corrmethod="both", crit="ICL", preout=True, postout=True),
+     dict(corr_method=2, criterion=1, pre_out=1, post_out=1)),
+    (80, dict(minclus=2, maxclus=3, corrmethod="spearman", crit="ICL"),
+     dict(min_clusters=2, max_clusters=3, corr_method=1, criterion=1)),
+    (60, dict(maxclus=5, corrmethod="pearson", crit="BIC", semantics="fixed", rand="lcg"),
+     dict(max_clusters=5, corr_method=0, criterion=0, semantics=1, rand_mode=1)),
+])
+def test_few_samples_run_full_waves_in_tiles(samples, gargs, oargs):
+    """With few samples the tile kernel is the faster one for a full wave (20 warps of 32 pairs on every SM), this one
+    for a part of it.  Both give the oracle's bits; the slices lie at a work block's start and at the wave's end."""
+    import torch
+    wave = torch.cuda.get_device_properties(0).multi_processor_count * 20 * 32
+    genes = 600
+    assert 32768 + wave <= genes * (genes - 1) // 2
+    gem = synthetic.generate(2, genes=genes, samples=samples)
+    kernel, whole = _slices(gem, gargs, oargs, 32768, wave, [(0, 200), (wave - 60, 60)])
+    assert kernel == "tiles"
+    kernel, part = _slices(gem, gargs, oargs, 32768, 3000, [])
+    assert kernel == "gmm pairs"
+    assert np.array_equal(whole.K[:3000], part.K)
+    assert np.array_equal(whole.labels[:3000][part.K > 1], part.labels[part.K > 1])
+    assert np.array_equal(whole.corr[:3000], part.corr, equal_nan=True)
