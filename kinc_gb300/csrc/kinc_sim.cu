@@ -889,7 +889,7 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
    const size_t slots = (size_t)grid * wpb;
    ctx->sms = prop.multiProcessorCount;
    ctx->n_cap = S;
-   if ( params->clus_method == 1 )
+   if ( params->clus_method == 1 || (params->clus_method == 0 && params->corr_method != 1 && params->precision == 0) )
    {
       /* usable counts: genes of every sample, and the largest of a gene */
       std::vector<int> usable((size_t)W * 32 + 1);
@@ -906,6 +906,9 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
       ctx->d_order = nullptr;
       ctx->n_cap = usable.back();
       for ( int i = 0; i < S; ++i ) ctx->n_mean += std::pow((double)usable[(size_t)i] / genes, 2.0);
+   }
+   if ( params->clus_method == 1 )
+   {
       ctx->gmm_per_sm = sim_gmm_pairs_per_sm(dp, ctx->n_cap);
       ctx->gmm_wave = (int64_t)slots * TILE;
    }
@@ -1031,10 +1034,12 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
    int launches = 0;
 
    const bool orders = ctx->orders.order != nullptr;      /* Spearman from the genes' orders counts by itself */
+   /* every Pearson run with the reference's packed-array reads needs the links */
+   const bool links = (dp.corr == 0 || dp.corr == 2) && dp.semantics == 0;
    if ( !orders || dp.corr == 2 )
    {
       k_count<<<(int)std::min<int64_t>((span + 255) / 256, 65535), 256, 0, st>>>(ctx->d_umask, ctx->W, lo, span,
-                                                                                  ctx->d_N, ctx->d_most32);
+                                                                                  ctx->d_N, links ? ctx->d_most32 : nullptr);
       ++launches;
    }
    if ( dp.clus != 0 && dp.rand_mode == 0 )
@@ -1059,9 +1064,8 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
       launches += 3;
       ctx->q_valid_end = end;
    }
-   if ( (dp.corr == 0 || dp.corr == 2) && dp.semantics == 0 )
+   if ( links )
    {
-      /* every Pearson run with the reference's packed-array reads needs the links */
       CK(launch_links(ctx->d_N, ctx->d_most32, span, ctx->d_pg, st));
       ++launches;
    }
@@ -1095,7 +1099,7 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
    ctx->last_kernel = KINC_SIM_KERNEL_GENES;
    if ( lanes )
    {
-      CK(sim_launch_pearson(ctx->sms, st, dp, ctx->dd, B));
+      CK(sim_launch_pearson(ctx->sms, st, dp, ctx->dd, B, ctx->n_mean));
       if ( orders )
       {
          launches += 2;

@@ -485,8 +485,8 @@ bool sim_gmm_pairs_better(const DevParams& P, int per_sm, double n, int64_t size
 size_t sim_gmm_pairs_scratch(int sms, const DevParams& P, int n_cap, char* base, DevScratch& W);
 cudaError_t sim_launch_gmm_pairs(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevScratch& W,
                                  const DevBlock& B, int n_cap);
-/* Pearson without clustering (sim_none.cu) */
-cudaError_t sim_launch_pearson(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B);
+/* Pearson without clustering (sim_none.cu); n: a pair's usable samples, on average */
+cudaError_t sim_launch_pearson(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B, double n);
 /* Spearman without clustering from every gene's sample order (sim_none.cu): whether these arguments run there,
  * the orders of a matrix (the bytes they take, laid out from base; and their kernel), and the launch
  * (tied_pairs: room for the block's pairs; B.tiles counts them, zero at first) */

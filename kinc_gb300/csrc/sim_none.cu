@@ -1,4 +1,4 @@
-/* Similarity without clustering (clusmethod none): Pearson with one thread per pair, Spearman from every
+/* Similarity without clustering (clusmethod none): Pearson from the rows of the matrix, Spearman from every
  * gene's sample order, and the tile kernel's specialisation for what is left. */
 #include "sim_pair.cuh"
 
@@ -130,28 +130,27 @@ static cudaError_t sim_launch_pearson_lanes(int sms, cudaStream_t st, const DevP
 }
 
 /*
- * The same for matrices of up to PT_WORDS * 32 samples, on tiles of 16 x 32 genes: the threads of a CTA
- * share the tile's values in shared memory, 32 samples at a time and zero where unusable, and each sums four
- * pairs (2 x 2 genes) in registers.  Which samples a pair adds is a bit mask per 32 samples: the usable ones,
- * or with semantics 0 those of them whose rank is itself a usable position (the r-th usable sample is read at
- * position r), so every addition is one predicated instruction.  The points that positions i >= N read follow:
- * the chain of earlier pairs with larger counts N_c, each giving its last N_c - i usable samples.
+ * The same on tiles of genes: the threads of a CTA share the tile's values in shared memory, 32 samples at a time and
+ * zero where unusable, and each sums R x R pairs (R genes x, R genes y) in registers.  Which samples a pair adds is a
+ * bit mask per 32 samples: the usable ones, or with semantics 0 those of them whose rank is itself a usable position
+ * (the r-th usable sample is read at position r), so every addition is one predicated instruction.  The points that
+ * positions i >= N read follow: the chain of earlier pairs with larger counts N_c, each giving its last N_c - i usable
+ * samples.
  *
- * One thread per pair straight from the matrix rows (k_pearson_lanes) issued 49 instructions per sample and
- * touched 32 rows per load; this one issues 9 to 11 (5 predicated additions, the bit test, the products) and
- * keeps 0.85 of the issue slots busy.  All pairs of 1,237 x 611 (semantics 1): 633 -> 200 us; of 1,000 x 200
- * (semantics 0): 375 -> 168 us with the launches before it, 45 % of it the points of earlier pairs.
+ * One thread per pair straight from the matrix rows (k_pearson_lanes) issues 49 instructions per sample and touches
+ * 32 rows per load.  R = 2 issues 9 to 11 (5 predicated additions, the bit test, the products) and keeps 0.85 of the
+ * issue slots busy; R = 1 issues more but has four times the threads, which blocks of few pairs, and the walks along
+ * the chain, need.  The choice and its times: sim_launch_pearson.
  */
 constexpr int PT_THREADS = 128;
-constexpr int PT_WORDS = 128;
 constexpr int PT_SMEM = 100 * 1024;         /* dynamic shared memory at most; the kernels' limit, the same for every caller
                                                (it belongs to the kernel, not to a context) */
 
-/* a tile of TX x (512 / TX) genes; few rows x take flat tiles */
-template <int TX>
+/* a tile of TX genes x and as many y as make R x R pairs a thread; few rows x take flat tiles */
+template <int TX, int R>
 struct PearsonTile
 {
-   static constexpr int X = TX, Y = 4 * PT_THREADS / TX;
+   static constexpr int X = TX, Y = R * R * PT_THREADS / TX;
    static constexpr int GENES = X + Y;
    static constexpr int ROW = GENES + 2;    /* floats between samples */
    static size_t bytes(int W) { return (size_t)(32 * ROW + GENES * W) * sizeof(float); }
@@ -176,6 +175,22 @@ struct PearsonSums
 {
    float x = 0.f, y = 0.f, xx = 0.f, yy = 0.f, xy = 0.f;
 };
+
+/* a thread's values of a sample and their squares */
+template <int R>
+__device__ __forceinline__ void pearson_values(const float* v, float (&x)[R], float (&xx)[R])
+{
+   if constexpr ( R == 2 )
+   {
+      const float2 q = *reinterpret_cast<const float2*>(v);
+      x[0] = q.x;
+      x[1] = q.y;
+   }
+   else
+      x[0] = *v;
+#pragma unroll
+   for ( int a = 0; a < R; ++a ) xx[a] = x[a] * x[a];
+}
 
 /* one sample added if bit `b` of `in` is set */
 __device__ __forceinline__ void pearson_add(PearsonSums& s, uint32_t in, int b, float vx, float vy, float vxx, float vyy,
@@ -248,12 +263,12 @@ __device__ inline void pearson_stale(const DevParams& P, const DevData& D, const
    /* beyond the longest of them the array still holds zeros, which change no sum */
 }
 
-template <int TX>
+template <int TX, int R>
 __global__ void __launch_bounds__(PT_THREADS)
 k_pearson_tiles(DevParams P, DevData D, DevBlock B, int x0)
 {
-   constexpr int PT_X = PearsonTile<TX>::X, PT_Y = PearsonTile<TX>::Y, PT_GENES = PearsonTile<TX>::GENES,
-                 PT_ROW = PearsonTile<TX>::ROW;
+   using T = PearsonTile<TX, R>;
+   constexpr int PT_X = T::X, PT_Y = T::Y, PT_GENES = T::GENES, PT_ROW = T::ROW;
    extern __shared__ __align__(16) float pt_smem[];
    float* v = pt_smem;                                            /* [32][PT_ROW] */
    uint32_t* mask = (uint32_t*)(pt_smem + 32 * PT_ROW);           /* [PT_GENES][W] */
@@ -266,7 +281,7 @@ k_pearson_tiles(DevParams P, DevData D, DevBlock B, int x0)
       if ( last < B.start || first >= B.start + B.size ) return;
    }
    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-   const int tx = 2 * (tid / (PT_Y / 2)), ty = 2 * (tid % (PT_Y / 2));
+   const int tx = R * (tid / (PT_Y / R)), ty = R * (tid % (PT_Y / R));
    auto gene = [&](int i) { return i < PT_X ? gx + i : gy + i - PT_X; };
    for ( int i = tid; i < PT_GENES * P.W; i += PT_THREADS )
    {
@@ -288,10 +303,17 @@ k_pearson_tiles(DevParams P, DevData D, DevBlock B, int x0)
    fetch(0);
    __syncthreads();
 
-   const uint32_t* mx[2] = { mask + tx * P.W, mask + (tx + 1) * P.W };
-   const uint32_t* my[2] = { mask + (PT_X + ty) * P.W, mask + (PT_X + ty + 1) * P.W };
-   PearsonSums sums[2][2];
-   int n[2][2] = { { 0, 0 }, { 0, 0 } };
+   const uint32_t *mx[R], *my[R];
+   PearsonSums sums[R][R];
+   int n[R][R];
+#pragma unroll
+   for ( int a = 0; a < R; ++a )
+   {
+      mx[a] = mask + (tx + a) * P.W;
+      my[a] = mask + (PT_X + ty + a) * P.W;
+#pragma unroll
+      for ( int b = 0; b < R; ++b ) n[a][b] = 0;
+   }
    for ( int w = 0; w < P.W; ++w )
    {
 #pragma unroll
@@ -302,11 +324,11 @@ k_pearson_tiles(DevParams P, DevData D, DevBlock B, int x0)
       }
       __syncthreads();
       if ( w + 1 < P.W ) fetch(w + 1);
-      uint32_t in[2][2];
+      uint32_t in[R][R];
 #pragma unroll
-      for ( int a = 0; a < 2; ++a )
+      for ( int a = 0; a < R; ++a )
 #pragma unroll
-         for ( int b = 0; b < 2; ++b )
+         for ( int b = 0; b < R; ++b )
          {
             const uint32_t u = mx[a][w] & my[b][w];
             uint32_t take = u;
@@ -321,21 +343,20 @@ k_pearson_tiles(DevParams P, DevData D, DevBlock B, int x0)
 #pragma unroll 8
       for ( int s = 0; s < 32; ++s )
       {
-         const float2 vx = *reinterpret_cast<const float2*>(v + s * PT_ROW + tx);
-         const float2 vy = *reinterpret_cast<const float2*>(v + s * PT_ROW + PT_X + ty);
-         const float xs[2] = { vx.x, vx.y }, ys[2] = { vy.x, vy.y };
-         const float xq[2] = { vx.x * vx.x, vx.y * vx.y }, yq[2] = { vy.x * vy.x, vy.y * vy.y };
+         float xs[R], ys[R], xq[R], yq[R];
+         pearson_values(v + s * PT_ROW + tx, xs, xq);
+         pearson_values(v + s * PT_ROW + PT_X + ty, ys, yq);
 #pragma unroll
-         for ( int a = 0; a < 2; ++a )
+         for ( int a = 0; a < R; ++a )
 #pragma unroll
-            for ( int b = 0; b < 2; ++b ) pearson_add(sums[a][b], in[a][b], s, xs[a], ys[b], xq[a], yq[b], xs[a] * ys[b]);
+            for ( int b = 0; b < R; ++b ) pearson_add(sums[a][b], in[a][b], s, xs[a], ys[b], xq[a], yq[b], xs[a] * ys[b]);
       }
       __syncthreads();
    }
 #pragma unroll
-   for ( int a = 0; a < 2; ++a )
+   for ( int a = 0; a < R; ++a )
 #pragma unroll
-      for ( int b = 0; b < 2; ++b )
+      for ( int b = 0; b < R; ++b )
       {
          const int x = gx + tx + a, y = gy + ty + b;
          if ( x >= P.G || y >= x ) continue;
@@ -354,19 +375,42 @@ k_pearson_tiles(DevParams P, DevData D, DevBlock B, int x0)
       }
 }
 
-template <int TX>
+template <int TX, int R>
 static cudaError_t launch_pearson_tiles(cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B, int x0,
                                         int x1)
 {
-   const int smem = (int)PearsonTile<TX>::bytes(P.W);
-   const cudaError_t e = cudaFuncSetAttribute(k_pearson_tiles<TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM);
+   using T = PearsonTile<TX, R>;
+   const int smem = (int)T::bytes(P.W);
+   /* 48 KB need no leave (the call costs a microsecond) */
+   const cudaError_t e = smem <= 48 * 1024 ? cudaSuccess
+      : cudaFuncSetAttribute(k_pearson_tiles<TX, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM);
    if ( e != cudaSuccess ) return e;
-   const dim3 grid((x1 + PearsonTile<TX>::Y - 1) / PearsonTile<TX>::Y, (x1 - x0) / TX + 1);
-   k_pearson_tiles<TX><<<grid, PT_THREADS, smem, st>>>(P, D, B, x0);
+   const dim3 grid((x1 + T::Y - 1) / T::Y, (x1 - x0) / TX + 1);
+   k_pearson_tiles<TX, R><<<grid, PT_THREADS, smem, st>>>(P, D, B, x0);
    return cudaGetLastError();
 }
 
-cudaError_t sim_launch_pearson(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B)
+/* whether the masks of a tile's genes fit in shared memory beside 32 samples of their values */
+template <int TX, int R>
+static bool pearson_tiles_fit(const DevParams& P)
+{
+   return PearsonTile<TX, R>::bytes(P.W) <= (size_t)PT_SMEM;
+}
+
+/*
+ * Microseconds, k_pearson_lanes / R = 1 / R = 2 (with the launches before them), by the mean N of a pair over S:
+ *   1,000 samples, own values      1 pair, 0.9: 81 / 51 / 122      500 pairs: 143 / 53 / 125     32,768: 154 / 44 / 73
+ *                                  131,072: 259 / 112 / 102        499,500: 899 / 326 / 260
+ *   1,000 samples, packed reads    1 pair, 0.9: 121 / 60 / 154     500 pairs: 393 / 80 / 193     32,768: 514 / 90 / 201
+ *                                  499,500, 0.9: 1,967 / 518 / 527    1,048,576: 3,837 / 1,001 / 940
+ *                                  32,768, 0.49: 1,713 / 683 / 2,093  1,048,576: 9,499 / 3,915 / 5,004
+ *   lanes pass over what a pair lacks, tiles do not: own values, 262,144 pairs, 0.25: 234 / 179 / 184; 0.04: 123 / 179 /
+ *   180; packed reads 0.25: 727 / 376 / 495, 0.04: 215 / 341 / 452; one pair, packed reads 0.49: 96 / 70 / 193, 0.25:
+ *   56 / 72 / 199.
+ * So lanes where a pair has less than an eighth of the samples (a few pairs: a third), R = 2 from 120,000 pairs with own
+ * values and from 900,000 with packed reads and little missing, R = 1 elsewhere.
+ */
+cudaError_t sim_launch_pearson(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B, double n)
 {
    /* the rows x of the block */
    auto row_of = [](int64_t p) {
@@ -376,10 +420,15 @@ cudaError_t sim_launch_pearson(int sms, cudaStream_t st, const DevParams& P, con
       return (int)x;
    };
    const int x0 = row_of(B.start), x1 = row_of(B.start + B.size - 1), rows = x1 - x0 + 1;
-   /* the masks of a tile's genes lie in shared memory beside 32 samples of their values */
-   if ( rows <= 2 && PearsonTile<2>::bytes(P.W) <= PT_SMEM ) return launch_pearson_tiles<2>(st, P, D, B, x0, x1);
-   if ( rows <= 8 && PearsonTile<4>::bytes(P.W) <= PT_SMEM ) return launch_pearson_tiles<4>(st, P, D, B, x0, x1);
-   if ( P.W <= PT_WORDS ) return launch_pearson_tiles<16>(st, P, D, B, x0, x1);
+   const double share = n / P.S;
+   if ( share < (B.size < 8 ? 0.35 : 0.125) ) return sim_launch_pearson_lanes(sms, st, P, D, B);
+   const bool many = P.semantics != 0 ? B.size >= 120000 : B.size >= 900000 && share >= 0.75;
+   if ( many && rows > 8 && pearson_tiles_fit<16, 2>(P) ) return launch_pearson_tiles<16, 2>(st, P, D, B, x0, x1);
+   if ( many && rows > 2 && pearson_tiles_fit<4, 2>(P) ) return launch_pearson_tiles<4, 2>(st, P, D, B, x0, x1);
+   /* tiles of 2 x 64, 4 x 32 or 8 x 16 genes */
+   if ( rows <= 2 && pearson_tiles_fit<2, 1>(P) ) return launch_pearson_tiles<2, 1>(st, P, D, B, x0, x1);
+   if ( rows <= 6 && pearson_tiles_fit<4, 1>(P) ) return launch_pearson_tiles<4, 1>(st, P, D, B, x0, x1);
+   if ( pearson_tiles_fit<8, 1>(P) ) return launch_pearson_tiles<8, 1>(st, P, D, B, x0, x1);
    return sim_launch_pearson_lanes(sms, st, P, D, B);
 }
 

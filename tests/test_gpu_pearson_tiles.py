@@ -67,3 +67,37 @@ def test_infinities(semantics):
 def test_more_samples_than_the_tiles_take(semantics):
     _check(_matrix(12, 4100, 2), semantics)
     _check(_matrix(12, 4096, 2), semantics)
+
+
+def _sparse(genes, samples, share, seed=5):
+    rng = np.random.default_rng(seed)
+    gem = rng.normal(8.0, 2.0, (genes, samples)).astype(np.float32)
+    gem[rng.random(gem.shape) >= share] = np.nan
+    return gem
+
+
+@pytest.mark.parametrize("semantics", ["reference", "fixed"])
+@pytest.mark.parametrize("gem,size", [
+    (_matrix(520, 40, 21), 130000),                  # many pairs: four a thread with own values, one with packed reads
+    (_matrix(1360, 34, 22, 0.02), 910000),           # and four a thread with packed reads
+    (_sparse(60, 90, 0.3), 1770),                    # a pair has a tenth of the samples: one thread per pair
+    (_sparse(60, 90, 0.45), 1770),                   # a fifth: tiles for many pairs, one thread per pair for a few
+    (_matrix(14, 6000, 23), 91),                     # more samples than fit beside 16 x 32 genes
+], ids=["130k", "910k", "sparse", "half", "6000"])
+def test_tile_choices(gem, size, semantics):
+    """Whole work blocks from the start; few rows and few pairs; the oracle on every part (for the largest on its last
+    work block, whose packed reads look back into that block only)."""
+    genes = gem.shape[0]
+    row = lambda x: x * (x - 1) // 2  # noqa: E731
+    sim = Similarity(gem, semantics=semantics, minsamp=2)
+    whole = sim.execute(None, start=0, size=size)
+    last = (size - 1) // 32768 * 32768
+    for start, n in [(last, size - last), (0, min(size, 500))]:
+        _, _, corr, _ = pyoracle.run_block(gem, pyoracle.params(semantics=int(semantics == "fixed"), min_samples=2), start, n)
+        assert np.array_equal(whole.corr[start:start + n], corr, equal_nan=True)
+    for start, n in [(row(genes - 3) + 1, 1), (row(genes - 3) + 2, 7), (row(genes - 5), 2 * genes - 12), (row(genes - 7) + 2, 4 * genes)]:
+        n = min(n, size - start)
+        if start < 0 or n < 1:
+            continue
+        assert np.array_equal(sim.execute(None, start=start, size=n).corr, whole.corr[start:start + n], equal_nan=True)
+    sim.close()
