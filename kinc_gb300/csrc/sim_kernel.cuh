@@ -488,16 +488,19 @@ cudaError_t sim_launch_gmm_pairs(int sms, cudaStream_t st, const DevParams& P, c
 /* Pearson without clustering (sim_none.cu); n: a pair's usable samples, on average */
 cudaError_t sim_launch_pearson(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B, double n);
 /* Spearman without clustering from every gene's sample order (sim_none.cu): whether these arguments run there,
- * the orders of a matrix (the bytes they take, laid out from base; and their kernel), and the launch
+ * the orders of a matrix (the bytes they take, laid out from base; their kernel, which also fills in the launches'
+ * sizes -- four queries of the runtime, 4 us of a call), and the launch
  * (tied_pairs: room for the block's pairs; B.tiles counts them, zero at first) */
 struct SpearmanOrders
 {
    uint16_t* order;                             /* [G][S] */
    uint8_t* ties;                               /* [G] */
+   int warp_bytes, per_sm;                      /* the walks: shared memory of a warp, CTAs an SM holds */
+   int net_bytes, net_per_sm;                   /* the networks of the tied pairs: of a CTA, CTAs an SM holds */
 };
 bool sim_spearman_orders_fit(const DevParams& P);
 size_t sim_spearman_orders_bytes(const DevParams& P, char* base, SpearmanOrders* out);
-cudaError_t sim_spearman_orders(cudaStream_t st, const DevParams& P, const DevData& D, const SpearmanOrders& R);
+cudaError_t sim_spearman_orders(cudaStream_t st, const DevParams& P, const DevData& D, SpearmanOrders& R);
 cudaError_t sim_launch_spearman(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B,
                                 const SpearmanOrders& R, int32_t* tied_pairs);
 SimKernel sim_kernel_gmm(int max_k, bool opencl);

@@ -517,17 +517,8 @@ bool sim_spearman_orders_fit(const DevParams& P)
 size_t sim_spearman_orders_bytes(const DevParams& P, char* base, SpearmanOrders* out)
 {
    const size_t order = ((size_t)P.G * P.S * sizeof(uint16_t) + 255) & ~(size_t)255;
-   if ( out ) *out = SpearmanOrders { (uint16_t*)base, (uint8_t*)(base + order) };
+   if ( out ) *out = SpearmanOrders { (uint16_t*)base, (uint8_t*)(base + order), 0, 0, 0, 0 };
    return order + (size_t)P.G;
-}
-
-cudaError_t sim_spearman_orders(cudaStream_t st, const DevParams& P, const DevData& D, const SpearmanOrders& R)
-{
-   const int smem = P.P2 * (int)sizeof(unsigned long long);
-   const cudaError_t e = cudaFuncSetAttribute(k_gene_order, cudaFuncAttributeMaxDynamicSharedMemorySize, ORDER_SMEM);
-   if ( e != cudaSuccess ) return e;
-   k_gene_order<<<std::min(P.G, 16384), ORDER_THREADS, smem, st>>>(D.gem, D.umask, P.G, P.S, P.W, P.P2, R.order, R.ties);
-   return cudaGetLastError();
 }
 
 /*
@@ -688,25 +679,35 @@ __global__ void __launch_bounds__(32) k_spearman_ties(DevParams P, DevData D, De
    }
 }
 
+cudaError_t sim_spearman_orders(cudaStream_t st, const DevParams& P, const DevData& D, SpearmanOrders& R)
+{
+   const int mask = (P.W * 4 + 15) & ~15;
+   R.warp_bytes = mask + ((P.S * 2 + 15) & ~15);
+   R.net_bytes = mask + 2 * P.P2 * (int)sizeof(float);
+   const int smem = P.P2 * (int)sizeof(unsigned long long);
+   cudaError_t e = cudaFuncSetAttribute(k_gene_order, cudaFuncAttributeMaxDynamicSharedMemorySize, ORDER_SMEM);
+   if ( e == cudaSuccess ) e = cudaFuncSetAttribute(k_spearman_orders, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEARMAN_SMEM);
+   if ( e == cudaSuccess ) e = cudaFuncSetAttribute(k_spearman_ties, cudaFuncAttributeMaxDynamicSharedMemorySize, TIES_SMEM);
+   if ( e == cudaSuccess )
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&R.per_sm, k_spearman_orders, SPEARMAN_WARPS * 32,
+                                                        (size_t)R.warp_bytes * SPEARMAN_WARPS);
+   if ( e == cudaSuccess ) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&R.net_per_sm, k_spearman_ties, 32, R.net_bytes);
+   if ( e != cudaSuccess ) return e;
+   k_gene_order<<<std::min(P.G, 16384), ORDER_THREADS, smem, st>>>(D.gem, D.umask, P.G, P.S, P.W, P.P2, R.order, R.ties);
+   return cudaGetLastError();
+}
+
 cudaError_t sim_launch_spearman(int sms, cudaStream_t st, const DevParams& P, const DevData& D, const DevBlock& B,
                                 const SpearmanOrders& R, int32_t* tied_pairs)
 {
-   const int mask = (P.W * 4 + 15) & ~15;
-   const int bytes = mask + ((P.S * 2 + 15) & ~15);
-   const int smem = bytes * SPEARMAN_WARPS, net = mask + 2 * P.P2 * (int)sizeof(float);
-   int per_sm = 1, net_per_sm = 1;
-   cudaError_t e = cudaFuncSetAttribute(k_spearman_orders, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEARMAN_SMEM);
-   if ( e == cudaSuccess ) e = cudaFuncSetAttribute(k_spearman_ties, cudaFuncAttributeMaxDynamicSharedMemorySize, TIES_SMEM);
-   if ( e == cudaSuccess )
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spearman_orders, SPEARMAN_WARPS * 32, smem);
-   if ( e == cudaSuccess ) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&net_per_sm, k_spearman_ties, 32, net);
-   if ( e != cudaSuccess ) return e;
-   int64_t grid = (int64_t)sms * std::max(1, per_sm);
+   int64_t grid = (int64_t)sms * std::max(1, R.per_sm);
    /* neighbouring pairs share x, so a warp takes up to 8 of them -- fewer if the warps would run out */
    const int per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(8, B.size / (grid * SPEARMAN_WARPS * 4)));
    grid = std::min(grid, (B.size + SPEARMAN_WARPS * per_warp - 1) / (SPEARMAN_WARPS * per_warp));
-   k_spearman_orders<<<(int)grid, SPEARMAN_WARPS * 32, smem, st>>>(P, D, B, R, tied_pairs, bytes, per_warp);
-   k_spearman_ties<<<(int)std::min<int64_t>(B.size, (int64_t)sms * std::max(1, net_per_sm)), 32, net, st>>>(P, D, B, tied_pairs);
+   k_spearman_orders<<<(int)grid, SPEARMAN_WARPS * 32, R.warp_bytes * SPEARMAN_WARPS, st>>>(P, D, B, R, tied_pairs, R.warp_bytes,
+                                                                                            per_warp);
+   k_spearman_ties<<<(int)std::min<int64_t>(B.size, (int64_t)sms * std::max(1, R.net_per_sm)), 32, R.net_bytes, st>>>(P, D, B,
+                                                                                                             tied_pairs);
    return cudaGetLastError();
 }
 
