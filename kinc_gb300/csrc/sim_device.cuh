@@ -223,15 +223,16 @@ __device__ __forceinline__ int next_pow2(int n)
 __device__ inline void warp_bitonic(int size, float* key, float* extra, int lane)
 {
    const int bsize = size / 2;
-   for ( int half = 1; half < size; half *= 2 )
+   for ( int ob = 2; ob <= size; ob *= 2 )
    {
-      for ( int t = half; t >= 1; t >>= 1 )
+      const int half = ob / 2;
+      for ( int ib = ob; ib >= 2; ib /= 2 )
       {
+         const int t = ib / 2;
          for ( int i = lane; i < bsize; i += 32 )
          {
-            /* a = i / t * 2t + i % t; powers of two, so no division */
-            const bool desc = (i & half) != 0;
-            const int a = 2 * i - (i & (t - 1));
+            const bool desc = (i / half) & 1;
+            const int a = (i / t) * ib + (i % t);
             const int b = a + t;
             const float ka = key[a];
             const float kb = key[b];
