@@ -273,7 +273,7 @@ __device__ __forceinline__ void gp_lds4(float4& v, uint32_t addr, int act)
 {
    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
                 : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
-                : "r"(addr), "r"(act));
+                : "r"(addr), "r"(act) : "memory");
 }
 
 /* acc + the first cnt (1..GP_CHUNK) floats at a 16-byte aligned shared-memory address, in order; 64 floats
@@ -285,7 +285,7 @@ __device__ __forceinline__ float gp_ordered_tail(uint32_t from, int cnt, float a
       for ( int g = 0; g < 4; ++g )
          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
                       : "=f"(q[g].x), "=f"(q[g].y), "=f"(q[g].z), "=f"(q[g].w)
-                      : "r"(at + 16 * g));
+                      : "r"(at + 16 * g) : "memory");
    };
    auto add16 = [&](const float4 (&q)[4]) {
 #pragma unroll

@@ -203,7 +203,7 @@ __device__ __forceinline__ void km_sweep(const KmStream& x, int j, int lim, int 
 #pragma unroll
          for ( int u = 0; u < U; ++u )
          {
-            asm volatile("ld.shared.b64 %0, [%1];" : "=l"(xv[u].v) : "r"(at + u * row));
+            asm volatile("ld.shared.b64 %0, [%1];" : "=l"(xv[u].v) : "r"(at + u * row) : "memory");
          }
          at += U * row;
          bool near = false;
