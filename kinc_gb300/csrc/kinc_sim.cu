@@ -623,23 +623,10 @@ extern "C" void kinc_sim_destroy(kinc_sim_ctx* ctx)
    delete ctx;
 }
 
-/* per warp slot scratch of K-means with a stream of pairs (kinc::k_kmeans_pairs) */
-struct KmPool
+/* K-means with a stream of pairs per warp (up to 5 clusters) */
+static bool streams_pairs(const kinc_sim_params& p, const SimKernel& k)
 {
-   int dmax = 0, tmax = 0, rs = 0;
-   size_t bytes = 0;
-};
-
-static KmPool km_pool_sizes(const kinc_sim_params& p, const SimKernel& k)
-{
-   KmPool m;
-   if ( p.clus_method != 2 || k.ks == 0 ) return m;
-   m.dmax = km_draws_per_pair(p.min_clusters, p.max_clusters);
-   m.tmax = TILE * (p.max_clusters - p.min_clusters + 1) * 10;
-   m.rs = k.ks == 3 ? km_record_floats<3>() : km_record_floats<5>();
-   m.bytes = (((size_t)m.dmax * TILE * sizeof(int32_t) + 255) & ~(size_t)255)
-             + (((size_t)m.tmax * m.rs * sizeof(float) + 255) & ~(size_t)255);
-   return m;
+   return p.clus_method == 2 && k.ks > 0;
 }
 
 /* K-means with local-memory centroids (more than 5 clusters) reads a contiguous copy of the lane's samples */
@@ -654,47 +641,84 @@ static bool gmm_in_pairs(const kinc_sim_ctx* ctx, int64_t size)
    return sim_gmm_pairs_better(ctx->dp, ctx->gmm_per_sm, ctx->n_mean, size, ctx->gmm_wave);
 }
 
-/* the scratch of the kernels that work in warp slots (32-pair tiles, and the K-means streams) */
+/* scratch of one warp slot, in bytes by array (DevScratch); 0: not used */
+struct SlotBytes
+{
+   size_t X = 0, lpx = 0, gam = 0, lbl = 0, wl = 0, ya = 0, yb = 0, yc = 0, rng = 0, sort = 0, Xl = 0, kmd = 0, kmr = 0;
+
+   size_t total() const
+   {
+      size_t sum = 0;
+      for ( size_t b : { X, lpx, gam, lbl, wl, ya, yb, yc, rng, sort, Xl, kmd, kmr } ) sum += (b + 255) & ~(size_t)255;
+      return sum;
+   }
+};
+
+/* sets P.km_dmax and P.km_tmax too */
+static SlotBytes slot_bytes(const kinc_sim_params& p, const SimKernel& k, DevParams& P, bool smem_sort)
+{
+   SlotBytes b;
+   const size_t col = (size_t)P.S * TILE;
+   b.sort = smem_sort ? 0 : (size_t)P.sort_floats * sizeof(float);
+   b.lpx = col * sizeof(float);
+   b.ya = col;
+   if ( streams_pairs(p, k) )
+   {
+      /* KM_COLS open pairs: their samples, labels, draws and the records of their runs; distances and labels of 32 runs
+       * at a time for the log-likelihoods */
+      P.km_dmax = km_draws_per_pair(p.min_clusters, p.max_clusters);
+      P.km_tmax = KM_COLS * (p.max_clusters - p.min_clusters + 1) * 10;
+      b.X = (size_t)P.S * KM_COLS * sizeof(float2);
+      b.lbl = (size_t)P.S * KM_COLS;
+      b.kmd = (size_t)P.km_dmax * KM_COLS * sizeof(int32_t);
+      b.kmr = (size_t)P.km_tmax * (k.ks == 3 ? km_record_floats<3>() : km_record_floats<5>()) * sizeof(float);
+      return b;
+   }
+   P.km_dmax = P.km_tmax = 0;
+   b.X = col * sizeof(float2);
+   b.gam = col * sizeof(float) * P.gam_k;
+   b.lbl = b.wl = b.yb = b.yc = col;
+   b.rng = (size_t)RNG_WORDS * TILE * sizeof(uint32_t);
+   b.Xl = lane_major(p, k) ? col * sizeof(float2) : 0;
+   return b;
+}
+
+/* the arrays of `slots` warp slots, from base + off on; off moves behind them */
+static DevScratch slot_arrays(const SlotBytes& b, size_t slots, void* base, size_t& off)
+{
+   auto take = [&](size_t bytes) -> void* {
+      if ( bytes == 0 ) return nullptr;
+      const size_t o = off;
+      off += (slots * bytes + 255) & ~(size_t)255;
+      return (void*)((uintptr_t)base + o);
+   };
+   DevScratch W {};
+   W.X = (float2*)take(b.X);
+   W.lpx = (float*)take(b.lpx);
+   W.gam = (float*)take(b.gam);
+   W.lbl = (int8_t*)take(b.lbl);
+   W.wl = (int8_t*)take(b.wl);
+   W.ya = (int8_t*)take(b.ya);
+   W.yb = (int8_t*)take(b.yb);
+   W.yc = (int8_t*)take(b.yc);
+   W.rng = (uint32_t*)take(b.rng);
+   W.sortbuf = (float*)take(b.sort);
+   W.Xl = (float2*)take(b.Xl);
+   W.kmd = (int32_t*)take(b.kmd);
+   W.kmr = (float*)take(b.kmr);
+   return W;
+}
+
+/* the context's scratch for the kernels that work in warp slots */
 static cudaError_t tile_scratch(kinc_sim_ctx* ctx)
 {
-   const size_t slots = (size_t)ctx->slots, col = (size_t)ctx->S * TILE;
-   const KmPool km = km_pool_sizes(ctx->params, ctx->kern);
-   size_t off = 0;
-   auto take = [&](size_t bytes) {
-      const size_t o = off;
-      off += (bytes + 255) & ~(size_t)255;
-      return o;
-   };
-   const size_t oX = take(slots * col * sizeof(float2));
-   const size_t oL = take(slots * col * sizeof(float));
-   const size_t oG = take(slots * col * sizeof(float) * ctx->dp.gam_k);
-   const size_t oB = take(slots * col);
-   const size_t oW = take(slots * col);
-   const size_t oA = take(slots * col);
-   const size_t oY = take(slots * col);
-   const size_t oC = take(slots * col);
-   const size_t oR = take(slots * RNG_WORDS * TILE * sizeof(uint32_t));
-   const size_t oS = take(ctx->smem_sort ? 0 : slots * ctx->dp.sort_floats * sizeof(float));
-   const bool xl = lane_major(ctx->params, ctx->kern);
-   const size_t oXl = take(xl ? slots * col * sizeof(float2) : 0);
-   const size_t oKd = take(slots * (size_t)km.dmax * TILE * sizeof(int32_t));
-   const size_t oKr = take(slots * (size_t)km.tmax * km.rs * sizeof(float));
-   const cudaError_t e = cudaMalloc(&ctx->d_scratch, off);
+   const SlotBytes b = slot_bytes(ctx->params, ctx->kern, ctx->dp, ctx->smem_sort);
+   size_t bytes = 0;
+   slot_arrays(b, (size_t)ctx->slots, nullptr, bytes);
+   const cudaError_t e = cudaMalloc(&ctx->d_scratch, bytes);
    if ( e != cudaSuccess ) return e;
-   char* base = (char*)ctx->d_scratch;
-   ctx->ds.X = (float2*)(base + oX);
-   ctx->ds.lpx = (float*)(base + oL);
-   ctx->ds.gam = ctx->dp.gam_k ? (float*)(base + oG) : nullptr;
-   ctx->ds.lbl = (int8_t*)(base + oB);
-   ctx->ds.wl = (int8_t*)(base + oW);
-   ctx->ds.ya = (int8_t*)(base + oA);
-   ctx->ds.yb = (int8_t*)(base + oY);
-   ctx->ds.yc = (int8_t*)(base + oC);
-   ctx->ds.rng = (uint32_t*)(base + oR);
-   ctx->ds.sortbuf = ctx->smem_sort ? nullptr : (float*)(base + oS);
-   ctx->ds.Xl = xl ? (float2*)(base + oXl) : nullptr;
-   ctx->ds.kmd = km.bytes ? (int32_t*)(base + oKd) : nullptr;
-   ctx->ds.kmr = km.bytes ? (float*)(base + oKr) : nullptr;
+   size_t off = 0;
+   ctx->ds = slot_arrays(b, (size_t)ctx->slots, ctx->d_scratch, off);
    return cudaSuccess;
 }
 
@@ -870,21 +894,15 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
    CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ctx->kern.fn, wpb * 32, ctx->smem_bytes));
    per_sm = std::max(1, per_sm);
 
-   /* scratch: per warp slot, interleaved by lane */
-   const size_t col = (size_t)S * TILE;
+   /* scratch: per warp slot */
    dp.gam_k = (KINC_STORE_GAMMA && params->clus_method == 1)
                  ? (params->max_clusters <= 3 ? 3 : params->max_clusters <= 5 ? 5 : 0) : 0;
-   const KmPool km = km_pool_sizes(*params, ctx->kern);
-   dp.km_dmax = km.dmax;
-   dp.km_tmax = km.tmax;
-   const size_t slot_bytes = col * sizeof(float2) * (lane_major(*params, ctx->kern) ? 2 : 1) + col * sizeof(float) * (1 + dp.gam_k)
-                             + 5 * col + (size_t)RNG_WORDS * TILE * sizeof(uint32_t)
-                             + (ctx->smem_sort ? 0 : sort_bytes_warp) + km.bytes + 256 * 10;
+   const size_t per_slot = slot_bytes(*params, ctx->kern, dp, ctx->smem_sort).total();
    size_t free_b = 0, total_b = 0;
    CKC(cudaMemGetInfo(&free_b, &total_b));
    int grid = prop.multiProcessorCount * per_sm;
    const size_t scratch_cap = free_b / 4;
-   while ( grid > prop.multiProcessorCount && (size_t)grid * wpb * slot_bytes > scratch_cap )
+   while ( grid > prop.multiProcessorCount && (size_t)grid * wpb * per_slot > scratch_cap )
       grid -= prop.multiProcessorCount;
    const size_t slots = (size_t)grid * wpb;
    ctx->sms = prop.multiProcessorCount;
@@ -1007,12 +1025,6 @@ extern "C" int kinc_sim_create(const float* gem, int32_t genes, int32_t samples,
 #undef CKC
 }
 
-/* K-means with a stream of pairs per warp (up to 5 clusters) */
-static bool streams_pairs(const kinc_sim_ctx* ctx)
-{
-   return ctx->params.clus_method == 2 && ctx->kern.ks > 0;
-}
-
 /* enqueue one device block [start, start+size) into device outputs; in_tiles: GMM in the tile kernel, whatever the
  * block's size */
 static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t* d_K, int8_t* d_labels,
@@ -1119,7 +1131,7 @@ static int enqueue_block(kinc_sim_ctx* ctx, int64_t start, int64_t size, int8_t*
    else
    {
       if ( !ctx->d_scratch ) return fail(ctx, KINC_SIM_ECUDA, "no scratch for a block of %lld pairs", (long long)size);
-      ctx->last_kernel = streams_pairs(ctx) ? KINC_SIM_KERNEL_KMEANS_PAIRS : KINC_SIM_KERNEL_TILES;
+      ctx->last_kernel = streams_pairs(ctx->params, ctx->kern) ? KINC_SIM_KERNEL_KMEANS_PAIRS : KINC_SIM_KERNEL_TILES;
       const SimKernel& k = ctx->kern;
       cudaError_t e = k.clus == 0 ? sim_launch_none(k, ctx->grid, ctx->smem_bytes, st, dp, ctx->dd, ctx->ds, B,
                                                     ctx->smem_sort)
@@ -1212,7 +1224,7 @@ std::string tune_key(const kinc_sim_ctx* ctx)
    const kinc_sim_params& p = ctx->params;
    char buf[400];
    snprintf(buf, sizeof buf, "kernel=%s clus=%d ks=%d ocl=%d corr=%d sem=%d pre=%d post=%d maxk=%d S<=%d gpu=%s sms=%d",
-            streams_pairs(ctx) ? "stream" : "tiles", p.clus_method, ctx->kern.ks, (int)ctx->kern.ocl, p.corr_method, p.semantics, p.pre_out, p.post_out,
+            streams_pairs(ctx->params, ctx->kern) ? "stream" : "tiles", p.clus_method, ctx->kern.ks, (int)ctx->kern.ocl, p.corr_method, p.semantics, p.pre_out, p.post_out,
             p.max_clusters, next_pow2_host(std::max(ctx->S, 2)), ctx->gpu_name, ctx->sms);
    for ( char* c = buf; *c; ++c )
       if ( *c == '\t' || *c == '\n' ) *c = ' ';
@@ -1344,7 +1356,7 @@ extern "C" int kinc_sim_autotune(kinc_sim_ctx* ctx, int64_t start, int64_t size,
    record(best, best_ms);
    const int warps_v[] = { 4, 8, 10, 16, 20 };
    const int pf_v[] = { 0, 4, 8, 16 };
-   const int passes = streams_pairs(ctx) ? 1 : 2;         /* one knob: one pass has timed all there is */
+   const int passes = streams_pairs(ctx->params, ctx->kern) ? 1 : 2;         /* one knob: one pass has timed all there is */
    for ( int pass = 0; pass < passes; ++pass )
    {
       const kinc_sim_launch start_best = best;
@@ -1356,7 +1368,7 @@ extern "C" int kinc_sim_autotune(kinc_sim_ctx* ctx, int64_t start, int64_t size,
           * 20 free-running warps from a 311,296-pair sample ran 1,048,576-pair blocks at 96k
           * pairs/s against 164k in rounds) */
          if ( knob == 2 && ctx->params.clus_method == 1 ) continue;
-         if ( knob != 1 && streams_pairs(ctx) ) continue;             /* its warps work apart and prefetch by their ring */
+         if ( knob != 1 && streams_pairs(ctx->params, ctx->kern) ) continue;             /* its warps work apart and prefetch by their ring */
          const int nv = knob == 0 ? 4 : knob == 1 ? 5 : 2;
          const kinc_sim_launch base = best;
          for ( int v = 0; v < nv; ++v )
@@ -1749,9 +1761,6 @@ extern "C" int kinc_sim_execute_block_noalloc(const float* d_gem, int32_t genes,
    }
    const size_t param_bytes_warp = (KINC_GMM_PARAMS_SMEM && kern.clus == 1 && kern.ks > 0)
                                       ? (size_t)7 * kern.ks * TILE * sizeof(float) : 0;
-   const KmPool km = km_pool_sizes(*params, kern);
-   dp.km_dmax = km.dmax;
-   dp.km_tmax = km.tmax;
    const int smem_sort = need_sort && param_bytes_warp == 0 && sort_bytes_warp * wpb <= 200 * 1024;
    const int smem_warp = (int)(warp_smem(kern, smem_sort ? sort_bytes_warp : 0) + param_bytes_warp);
    dp.smem_floats = smem_warp / (int)sizeof(float);
@@ -1776,46 +1785,17 @@ extern "C" int kinc_sim_execute_block_noalloc(const float* d_gem, int32_t genes,
    const size_t oQ = take((size_t)size * sizeof(uint64_t));
    const size_t oBsum = take((size_t)(nscan + 1) * sizeof(unsigned long long));
    const size_t oSmall = take(8 * sizeof(unsigned long long));
-   const size_t col = (size_t)S * TILE;
-   const size_t slot_bytes = ((col * sizeof(float2) + 255) & ~(size_t)255) + ((col * sizeof(float) + 255) & ~(size_t)255)
-                             + ((col * sizeof(float) * dp.gam_k + 255) & ~(size_t)255)
-                             + 5 * ((col + 255) & ~(size_t)255)
-                             + (((size_t)RNG_WORDS * TILE * sizeof(uint32_t) + 255) & ~(size_t)255)
-                             + (smem_sort ? 0 : ((sort_bytes_warp + 255) & ~(size_t)255))
-                             + ((params->clus_method == 2 && KINC_KMEANS_LANE_MAJOR && kern.ks == 0)
-                                   ? ((col * sizeof(float2) + 255) & ~(size_t)255) : 0)
-                             + km.bytes;
-   if ( off >= NOALLOC_SCRATCH_BYTES || (NOALLOC_SCRATCH_BYTES - off) / slot_bytes < (size_t)wpb )
+   const SlotBytes slot = slot_bytes(*params, kern, dp, smem_sort);
+   const size_t per_slot = slot.total();
+   if ( off >= NOALLOC_SCRATCH_BYTES || (NOALLOC_SCRATCH_BYTES - off) / per_slot < (size_t)wpb )
       return fail(nullptr, KINC_SIM_EINVAL,
                   "%d genes x %d samples and %lld pairs do not fit the %zu-byte allocation-free scratch",
                   genes, samples, (long long)size, NOALLOC_SCRATCH_BYTES);
-   const size_t nslots = ((NOALLOC_SCRATCH_BYTES - off) / slot_bytes) / wpb * wpb;
+   const size_t nslots = ((NOALLOC_SCRATCH_BYTES - off) / per_slot) / wpb * wpb;
    unsigned char* base = nd.scratch;
-   DevScratch ds {};
-   {
-      size_t o = off;
-      auto carve = [&](size_t bytes) {
-         unsigned char* p = base + o;
-         o += (bytes + 255) & ~(size_t)255;
-         return p;
-      };
-      ds.X = (float2*)carve(nslots * col * sizeof(float2));
-      ds.lpx = (float*)carve(nslots * col * sizeof(float));
-      ds.gam = dp.gam_k ? (float*)carve(nslots * col * sizeof(float) * dp.gam_k) : nullptr;
-      ds.lbl = (int8_t*)carve(nslots * col);
-      ds.wl = (int8_t*)carve(nslots * col);
-      ds.ya = (int8_t*)carve(nslots * col);
-      ds.yb = (int8_t*)carve(nslots * col);
-      ds.yc = (int8_t*)carve(nslots * col);
-      ds.rng = (uint32_t*)carve(nslots * RNG_WORDS * TILE * sizeof(uint32_t));
-      ds.sortbuf = smem_sort ? nullptr : (float*)carve(nslots * sort_bytes_warp);
-      ds.Xl = (params->clus_method == 2 && KINC_KMEANS_LANE_MAJOR && kern.ks == 0)
-                 ? (float2*)carve(nslots * col * sizeof(float2)) : nullptr;
-      ds.kmd = km.bytes ? (int32_t*)carve(nslots * (size_t)km.dmax * TILE * sizeof(int32_t)) : nullptr;
-      ds.kmr = km.bytes ? (float*)carve(nslots * (size_t)km.tmax * km.rs * sizeof(float)) : nullptr;
-      if ( o > NOALLOC_SCRATCH_BYTES )
-         return fail(nullptr, KINC_SIM_EINVAL, "allocation-free scratch layout overflow");
-   }
+   size_t used = off;
+   const DevScratch ds = slot_arrays(slot, nslots, base, used);
+   if ( used > NOALLOC_SCRATCH_BYTES ) return fail(nullptr, KINC_SIM_EINVAL, "allocation-free scratch layout overflow");
    uint32_t* d_umask = (uint32_t*)(base + oMask);
    double* d_logn = (double*)(base + oLogn);
    int32_t* d_N = (int32_t*)(base + oN);

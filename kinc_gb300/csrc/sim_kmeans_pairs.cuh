@@ -351,16 +351,16 @@ k_kmeans_pairs(DevParams P, DevData D, DevScratch W, DevBlock B, int smem_sort)
    const int lane = threadIdx.x & 31;
    const int warp = threadIdx.x >> 5;
    const int64_t slot = blockIdx.x * (int64_t)(blockDim.x >> 5) + warp;
-   const size_t tile = (size_t)P.S * TILE;
+   const size_t tile = (size_t)P.S * TILE, open_pairs = (size_t)P.S * KM_COLS;
    const int kmin = P.min_k, kmax = P.max_k;
    const int runs = 10 * (kmax - kmin + 1);               /* of one pair */
    const int sweeps = kmin == 1 ? runs - 10 : runs;       /* of them with more than one cluster */
 
-   float2* X = W.X + slot * tile;
-   int8_t* labels = W.lbl + slot * tile;
+   float2* X = W.X + slot * open_pairs;
+   int8_t* labels = W.lbl + slot * open_pairs;
    float* dbuf = W.lpx + slot * tile + lane;
    int8_t* ya = W.ya + slot * tile + lane;
-   int32_t* draws = W.kmd + (size_t)slot * P.km_dmax * TILE;
+   int32_t* draws = W.kmd + (size_t)slot * P.km_dmax * KM_COLS;
    float* rec = W.kmr + (size_t)slot * P.km_tmax * RS;
    float* ring = smem + (size_t)warp * P.smem_floats;
    float* sort = smem_sort ? ring : W.sortbuf + slot * (size_t)P.sort_floats;

@@ -66,3 +66,25 @@ def test_infinite_and_constant_genes():
     gem[5] *= np.float32(1e-25)
     _check(gem, dict(crit="ICL", corrmethod="spearman", postout=True, maxclus=4),
            dict(criterion=1, corr_method=1, post_out=1, max_clusters=4))
+
+
+def test_scratch_is_what_the_kernel_uses():
+    """A warp slot holds eight open pairs (samples, labels, draws, records of the runs) and the distances and labels of
+    32 runs, not 32 pairs: the worker takes that and no more (64 MB for everything else)."""
+    import torch
+    S, runs, draws, record = 4000, 30, 60, 4 * 3 + 1
+    gem = synthetic.generate(4, genes=40, samples=S)
+
+    def taken(matrix):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        sim = Similarity(matrix, clusmethod="kmeans", corrmethod="pearson", maxclus=3, crit="BIC")
+        sim.execute(None, start=0, size=100)
+        after = torch.cuda.mem_get_info()[0]
+        sim.close()
+        return before - after
+
+    taken(gem[:, :50])                                     # modules and runtime buffers
+    slots = torch.cuda.get_device_properties(0).multi_processor_count * 16
+    slot = 8 * (S * (8 + 1) + 4 * draws + 4 * record * runs) + 32 * S * (4 + 1)
+    assert taken(gem) <= slots * (slot + 4096) + (64 << 20)
