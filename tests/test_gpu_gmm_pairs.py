@@ -133,3 +133,24 @@ def test_few_samples_run_full_waves_in_tiles(samples, gargs, oargs):
     assert np.array_equal(whole.K[:3000], part.K)
     assert np.array_equal(whole.labels[:3000][part.K > 1], part.labels[part.K > 1])
     assert np.array_equal(whole.corr[:3000], part.corr, equal_nan=True)
+
+
+@pytest.mark.parametrize("genes,samples,gargs,oargs", [
+    # 16 warps a CTA, responsibilities in shared memory
+    (72, 150, dict(crit="BIC", corrmethod="spearman", preout=True, postout=True), dict(criterion=0, corr_method=1, pre_out=1, post_out=1)),
+    (72, 60, dict(crit="ICL", corrmethod="pearson", minclus=4, maxclus=4), dict(criterion=1, corr_method=0, min_clusters=4, max_clusters=4)),
+    (64, 190, dict(crit="ICL", corrmethod="both", minclus=5, maxclus=5), dict(criterion=1, corr_method=2, min_clusters=5, max_clusters=5)),
+    # 12 warps, in shared memory; 16 and 12 in global memory
+    (64, 300, dict(crit="BIC", corrmethod="pearson", minclus=4, maxclus=5), dict(criterion=0, corr_method=0, min_clusters=4, max_clusters=5)),
+    (64, 480, dict(crit="BIC", corrmethod="pearson", minclus=4, maxclus=5), dict(criterion=0, corr_method=0, min_clusters=4, max_clusters=5)),
+    (64, 900, dict(crit="ICL", corrmethod="pearson", minclus=5, maxclus=5), dict(criterion=1, corr_method=0, min_clusters=5, max_clusters=5)),
+])
+def test_more_pairs_than_twelve_an_sm(genes, samples, gargs, oargs):
+    """Blocks of more than 12 pairs an SM, where the number of warps is chosen by the samples; the oracle on the first
+    and the last pairs."""
+    gem = synthetic.generate(2, genes=genes, samples=samples)
+    total = genes * (genes - 1) // 2
+    import torch
+    assert total > 12 * torch.cuda.get_device_properties(0).multi_processor_count
+    kernel, _ = _slices(gem, gargs, oargs, 0, total, [(0, 100), (total - 30, 30)])
+    assert kernel == "gmm pairs"
