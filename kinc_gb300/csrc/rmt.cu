@@ -340,7 +340,9 @@ int device_setup(RmtDevice& d, int32_t G, int32_t K, int64_t n, const int32_t* x
       if ( x[i] <= y[i] || y[i] < 0 || x[i] >= G || c[i] < 0 || c[i] >= K )
          return rmt_fail(KINC_SIM_EINVAL, "item %lld (%d, %d, %d) outside %d genes x %d clusters", (long long)i, x[i],
                          y[i], c[i], G, K);
-   d.infinite = std::any_of(r, r + n, [](float v) { return std::isinf(v); });
+   int infinite = 0;                                     /* no early end: this loop is vectorised */
+   for ( int64_t i = 0; i < n; ++i ) infinite |= std::fabs(r[i]) > std::numeric_limits<float>::max();
+   d.infinite = infinite != 0;
    d.G = G;
    d.K = K;
    d.n = n;
@@ -570,7 +572,8 @@ int device_eigenvalues(RmtDevice& d, float t, std::vector<float>& eig, int32_t& 
       const int smem = (int)rmt_block_bytes(most[wide]);
       RCK(cudaMemcpyAsync(to, list[wide].data(), (size_t)count * sizeof(int32_t), cudaMemcpyHostToDevice, d.st));
       /* the kernel's limit, the same for every caller (it belongs to the kernel, not to a call) */
-      RCK(cudaFuncSetAttribute(k_rmt_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rmt_block_bytes(RMT_BLOCK)));
+      if ( smem > 48 * 1024 )
+         RCK(cudaFuncSetAttribute(k_rmt_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rmt_block_bytes(RMT_BLOCK)));
       k_rmt_blocks<<<count, wide ? RMT_BLOCK : RMT_BLOCK_WARP, smem, d.st>>>(d.dcomp, to, count, d.dA, d.dW);
       RCK(cudaGetLastError());
       to += count;
