@@ -653,7 +653,7 @@ def main():
     t0 = time.perf_counter()
     chosen, timed = sim.autotune(use_cache=not args.no_tune_cache)
     autotune = {"chosen": chosen, "candidates": timed, "seconds": time.perf_counter() - t0,
-                "sample_pairs": 4 * 32 * 16 * 152, "from_cache": len(timed) == 0}
+                "sample_pairs_at_most": 4 * 32 * 16 * 152, "from_cache": len(timed) == 0}
     dK = torch.empty(B, dtype=torch.int8, device="cuda")
     dL = torch.empty((B, S), dtype=torch.int8, device="cuda")
     dC = torch.empty((B, maxk), dtype=torch.float32, device="cuda")

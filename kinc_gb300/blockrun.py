@@ -95,7 +95,8 @@ def main(argv=None):
 
 
 def tune_grid(sim, args):
-    """The autotuner's pick against every launch shape, on the sample block it times."""
+    """The autotuner's pick against every launch shape of the kernel that runs the sample block (with GMM, a
+    block of this size may run in a kernel that takes no shape: then there is no grid)."""
     import time
 
     import torch
@@ -115,10 +116,19 @@ def tune_grid(sim, args):
     dL = torch.empty((size, S), dtype=torch.int8, device="cuda")
     dC = torch.empty((size, sim.params.max_clusters * nc), dtype=torch.float32, device="cuda")
     stream = torch.cuda.Stream()
+    default = sim.launch()
+    def execute():
+        _native.check(L.kinc_sim_execute_block_device(sim._ctx, start, size, vp(dK.data_ptr()), vp(dL.data_ptr()),
+                                                      vp(dC.data_ptr()), vp(stream.cuda_stream)), sim._ctx)
+        torch.cuda.synchronize()
+
+    execute()
+    kernel = sim.last_kernel()
+    rounds, prefetches = ((0, 1), (0, 4, 8, 16)) if kernel == "tiles" else ((default["rounds"],), (default["prefetch"],))
     grid = {}
-    for w in warps:
-        for r in (0, 1):
-            for pf in (0, 4, 8, 16):
+    for w in warps if kernel in ("tiles", "kmeans pairs") else ():
+        for r in rounds:
+            for pf in prefetches:
                 sim.set_launch(w, r, pf)
                 e0 = torch.cuda.Event(enable_timing=True)
                 e1 = torch.cuda.Event(enable_timing=True)
@@ -129,12 +139,14 @@ def tune_grid(sim, args):
                 e1.record(stream)
                 torch.cuda.synchronize()
                 grid[f"{w},{r},{pf}"] = e0.elapsed_time(e1)
-    best = min(grid, key=grid.get)
     pick = f"{chosen['warps_per_cta']},{chosen['rounds']},{chosen['prefetch']}"
-    print(json.dumps({"workload": args.workload, "genes": int(G), "samples": int(S),
-                      "sample_pairs": size, "autotune_s": tune_s, "autotune_candidates": len(cands),
-                      "picked": pick, "picked_ms": grid[pick], "best": best, "best_ms": grid[best],
-                      "picked_over_best": grid[pick] / grid[best], "grid_ms": grid}), flush=True)
+    out = {"workload": args.workload, "genes": int(G), "samples": int(S), "sample_pairs": size, "kernel": kernel,
+           "autotune_s": tune_s, "autotune_candidates": len(cands), "picked": pick}
+    if grid:
+        best = min(grid, key=grid.get)
+        out.update(picked_ms=grid[pick], best=best, best_ms=grid[best], picked_over_best=grid[pick] / grid[best],
+                   grid_ms=grid)
+    print(json.dumps(out), flush=True)
 
 
 if __name__ == "__main__":
