@@ -15,8 +15,8 @@
  * The pruned matrix is built on the GPU from the CMX items (no dense
  * genes x genes x clusters copy) and its eigenvalues are those of its connected
  * components (up to 128 rows: this library's kernel, Householder and bisection;
- * larger: cuSOLVER's symmetric eigensolver), in double precision, as the
- * reference's solver works in double; the unfolding (Akima spline) and the chi-square run on the host.
+ * larger ones, and matrices that are mostly one component: cuSOLVER's symmetric
+ * eigensolver), in double precision, as the reference's solver works in double; the unfolding (Akima spline) and the chi-square run on the host.
  */
 #ifndef KINC_RMT_H
 #define KINC_RMT_H

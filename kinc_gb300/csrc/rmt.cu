@@ -7,7 +7,8 @@
  * from the items into a dense double array in HBM, and their eigenvalues
  * (computeEigenvalues, :252-282, which solves the same double matrix): one
  * kernel for all components of up to 128 rows, cuSOLVER's symmetric
- * divide-and-conquer solver for each larger one.
+ * divide-and-conquer solver for larger ones, or for all rows together where that
+ * costs no more (rmt_plan).
  *
  * Host: the eigenvalues sorted by ascending |lambda| and converted to float,
  * the unique values (degenerate, :374-388), the Akima-spline unfolding

@@ -24,8 +24,9 @@
  * What bounds it: per 64 samples, component and iteration the fit needs 122
  * cycles of a scheduler's FP32 pipe (a packed FP32 instruction takes two; the
  * three exponentials are half of it) and the ordered sums 128 per fit; at K = 5
- * and N = 832 that is 192 cycles per SM and chunk against 323 measured with 11
- * pairs per SM.  The shared-memory pipe carries 26 wavefronts per component
+ * and N = 832 that is 192 cycles per SM and chunk of 64 samples, 59 % of the 323
+ * measured with 11 pairs per SM.  (Over a whole block, with its other K, sorts and
+ * waits, the counters show the FP32 pipe busy 43 % of the time.)  The shared-memory pipe carries 26 wavefronts per component
  * beside it.
  */
 #pragma once
