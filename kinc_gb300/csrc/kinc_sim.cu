@@ -1338,7 +1338,15 @@ extern "C" int kinc_sim_autotune(kinc_sim_ctx* ctx, int64_t start, int64_t size,
    } borrowed;
    if ( !ctx->d_scratch )
    {
-      CK(tile_scratch(ctx));
+      const cudaError_t e = tile_scratch(ctx);
+      if ( e == cudaErrorMemoryAllocation )
+      {
+         /* no room for a kernel that this worker does not run: its shape stays as it is */
+         cudaGetLastError();
+         if ( chosen ) *chosen = best;
+         return KINC_SIM_OK;
+      }
+      CK(e);
       borrowed.ctx = ctx;
       size = std::min(size, ctx->gmm_wave);
    }
