@@ -361,7 +361,6 @@ int device_setup(RmtDevice& d, int32_t G, int32_t K, int64_t n, const int32_t* x
    RCK(cudaMalloc(&d.dlist, rows * sizeof(int32_t)));
    RCK(cudaMalloc(&d.dplace, rows * sizeof(int2)));
    RCK(cudaMalloc(&d.dcomp, rows * sizeof(RmtComponent)));
-   RCK(cudaMalloc(&d.dinfo, sizeof(int32_t)));
    RCK(cudaMalloc(&d.dW, rows * sizeof(double)));
    if ( n > 0 )
    {
@@ -459,6 +458,7 @@ int large_matrix(RmtDevice& d, const RmtComponent& q)
    if ( !d.solver && (cusolverDnCreate(&d.solver) != CUSOLVER_STATUS_SUCCESS
                       || cusolverDnSetStream(d.solver, d.st) != CUSOLVER_STATUS_SUCCESS) )
       return rmt_fail(KINC_SIM_ECUDA, "cannot create the eigensolver");
+   if ( !d.dinfo ) RCK(cudaMalloc(&d.dinfo, sizeof(int32_t)));
    /* row-major with the lower triangle set = column-major with the upper triangle set */
    const int32_t m = q.size;
    double* A = d.dA + q.at;
