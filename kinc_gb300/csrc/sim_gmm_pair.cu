@@ -25,8 +25,8 @@ int sim_gmm_pairs_per_sm(const DevParams& P, int n_cap)
  *
  *  - Few samples: the updates between the iterations (123 in units of the tile kernel's sample and component) and
  *    what a sample takes besides its components outweigh the tile kernel's k n.  Measured / this formula, blocks of
- *    389,120 pairs, Pearson: k <= 2 n = 40: 0.51 / 0.51, 97: 0.79 / 0.80, 243: 1.08 / 1.11; k <= 3 n = 63:
- *    0.69 / 0.71; k <= 5 n = 40: 0.65 / 0.67, 63: 0.88 / 0.84, 97: 1.04 / 1.00, 162: 1.18 / 1.16.  One cluster
+ *    389,120 pairs (four waves and 10 / n), Pearson: k <= 2 n = 40: 0.51 / 0.47, 97: 0.79 / 0.77, 243: 1.08 / 1.06;
+ *    k <= 3 n = 63: 0.69 / 0.71; k <= 5 n = 40: 0.65 / 0.69, 63: 0.88 / 0.85, 97: 1.04 / 1.00, 162: 1.18 / 1.15.  One cluster
  *    takes two iterations, so the pair's other work decides: n = 40: 0.39 (with outliers and Spearman 0.67), 97:
  *    0.52 (0.88), 243: 0.79 (1.29), 810: 0.93 (1.60), and without sorts at most 0.84 in ten waves.
  *  - Many samples: fewer pairs fit an SM.  97,280 pairs of the 10 %-missing mixture workload, k <= 5, Spearman with
